@@ -12,7 +12,8 @@
 //           with all 32 lanes (the (p, element) pairs are flattened across the warp
 //           with a prefix sum, so list lengths never idle lanes), and each element
 //           is looked up in S(a).
-//  * undirected graph (forward CSR == reverse CSR): degree-ordered orientation
+//  * undirected graph (forward CSR == reverse CSR): in rank order (sp_tc_rank.cuh) by
+//    default; the anchor loops here, chosen by knob or on small graphs, use the orientation
 //    E+ = {(u,v): (deg u, u) < (deg v, v)}; a = u, S = P = N+(u), L(v) = N+(v).
 //    Each triangle is counted once, which equals the formula on a symmetric graph.
 //  * any other graph: the formula literally; a = v, S = N(v) ∩ (v, inf),
@@ -36,6 +37,7 @@
 #include <vector>
 
 #include "sp_internal.cuh"
+#include "sp_tc_rank.cuh"
 
 namespace sp {
 
@@ -685,6 +687,7 @@ __global__ void k_new_edges(const int32_t* __restrict__ off, const int32_t* __re
 }  // namespace tc
 
 struct TcPlan {
+  tcr::Plan rank;            // symmetric graphs: lists in rank order
   dbuf<int32_t> ooff, oadj;  // oriented CSR (undirected graphs)
   dbuf<int32_t> order;       // anchors, heaviest first
   dbuf<int> heavy;
@@ -714,17 +717,11 @@ void free_tc_plan(TcPlan* p) {
 
 static int build_tc_plan(sp_graph* g) {
   if (g->tc && g->tc->built) return SP_OK;
-  if (g->tc) {
-    free_tc_plan(g->tc);
-    g->tc = nullptr;
-  }
   SP_TRY(ensure_symmetry(g));
-  TcPlan* p = new TcPlan();
+  if (!g->tc) g->tc = new TcPlan();
+  TcPlan* p = g->tc;
   cudaStream_t s = g->stream;
-  auto fail = [&](int st) {
-    free_tc_plan(p);
-    return st;
-  };
+  auto fail = [&](int st) { return st; };  // what was built is kept; a later call builds again
   int st;
   if ((st = p->heavy.alloc(g->V)) || (st = p->ctr.alloc(2)) || (st = p->total.alloc(1))) return fail(st);
   if (g->symmetric == 1) {
@@ -782,8 +779,13 @@ static int build_tc_plan(sp_graph* g) {
     }
   }
   p->built = true;
-  g->tc = p;
   return SP_OK;
+}
+
+// The plan of counting in rank order (symmetric graphs; the symmetry must be known).
+static int build_rank_plan(sp_graph* g) {
+  if (!g->tc) g->tc = new TcPlan();
+  return tcr::build(g, g->tc->rank);
 }
 
 static tc::Lists tc_lists(sp_graph* g, int n) {
@@ -881,22 +883,56 @@ static int tc_variant_pick(sp_graph* g, int* cand) {
   return SP_OK;
 }
 
+// Items part, part + nparts, ... of the rank plan: the triangle count, or (counts given)
+// every vertex's count of those triangles, overwritten.
+static int rank_count(sp_graph* g, int part, int nparts, int64_t* triangle_count, int* counts) {
+  tcr::Plan& P = g->tc->rank;
+  cudaStream_t s = g->stream;
+  tcr::Args a;
+  a.oadj = P.oadj.p;
+  a.tasks = P.tasks.p;
+  a.tu = P.tu.p;
+  a.items = P.items.p;
+  a.itemv = P.itemv.p;
+  a.n_items = (const int32_t*)(P.out.p + tcr::OUT_ITEMS);
+  a.part = part;
+  a.nparts = nparts;
+  a.total = P.out.p;
+  a.next = (unsigned int*)(P.out.p + 16);
+  a.cf = P.cf.p;
+  const int most = P.items_max / nparts + 1;  // items of the part, at most
+  SP_CHECK_CUDA(cudaMemsetAsync(P.out.p, 0, tcr::OUT_ITEMS * sizeof(unsigned long long), s));
+  if (counts) {  // per vertex
+    constexpr int NW = tcr::PW;
+    constexpr size_t sm = tcr::smem_bytes(NW, true);
+    if (g->V) SP_CHECK_CUDA(cudaMemsetAsync(P.cf.p, 0, sizeof(int) * g->V, s));
+    auto k = tcr::k_count<true, NW, tcr::PMINB, tcr::PU>;
+    SP_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k<<<std::min(num_sms() * tcr::PMINB, (most + NW - 1) / NW), NW * 32, sm, s>>>(a);
+    SP_CHECK_LAUNCH();
+    if (g->V) {
+      tcr::k_by_vertex<<<std::min(num_sms() * 8, (g->V + 255) / 256), 256, 0, s>>>(g->V, P.order.p, P.cf.p, counts);
+      SP_CHECK_LAUNCH();
+    }
+    return SP_OK;
+  }
+  constexpr int NW = tcr::CW;
+  tcr::k_count<false, NW, tcr::CMINB, tcr::CU>
+      <<<std::min(num_sms() * tcr::CMINB, (most + NW - 1) / NW), NW * 32, tcr::smem_bytes(NW, false), s>>>(a);
+  SP_CHECK_LAUNCH();
+  unsigned long long h = 0;
+  SP_TRY(copy_out(&h, P.out.p, sizeof(h), s));
+  *triangle_count = (int64_t)h;
+  return SP_OK;
+}
+
 // Triangles anchored at order[0 .. n) (the whole count when order is the plan's and n = V).
-static int tc_count(sp_graph* g, const int32_t* order, int n, int64_t* triangle_count) {
+static int tc_count(sp_graph* g, const int32_t* order, int n, int cta_warps, int wu, int64_t* triangle_count) {
   TcPlan* p = g->tc;
   cudaStream_t s = g->stream;
   const tc::Lists L = tc_lists(g, n);
   SP_CHECK_CUDA(cudaMemsetAsync(p->ctr.p, 0, sizeof(unsigned int) * 2, s));
   SP_CHECK_CUDA(cudaMemsetAsync(p->total.p, 0, sizeof(unsigned long long), s));
-  int cta_warps = g->tc_cta_warps >= 0 ? g->tc_cta_warps : tc::CTA_WARPS_DEFAULT;
-  int wu = g->tc_unroll > 0 ? g->tc_unroll : tc::WU_DEFAULT;
-  int cand = -1;
-  SP_TRY(tc_variant_pick(g, &cand));
-  if (cand >= 0) {
-    if (tc::VARIANTS[cand].bitmap) cta_warps = tc::VARIANTS[cand].cta_warps;
-    else wu = tc::VARIANTS[cand].wu;
-  }
-  g->last_variant[VAR_TC] = cand;
   if (g->V <= 65536 && cta_warps > 0) {
     void (*k)(tc::Lists, const int32_t*, unsigned long long*, int*) =
         cta_warps == 2   ? tc::k_tc_bitmap_cta<2, 24, false>
@@ -961,6 +997,57 @@ static int order_part(sp_graph* g, int part, int nparts, dbuf<int32_t>& out, int
   return SP_OK;
 }
 
+// Up to this many entries a symmetric graph of at most 65536 vertices is counted by
+// k_tc_bitmap_cta: both take a call's own time of about 30 us there (R-MAT 13 of edge
+// factor 8, 115 thousand entries: 33 against 30), and its plan is made in fewer launches
+// (a first call 223 against 272 us).
+constexpr int64_t RANK_MIN_E = 1 << 17;
+
+// The triangles of part `part` of `nparts`. Symmetric graphs count in rank order
+// (sp_tc_rank.cuh, with the times of both) unless a knob or variant asks for a kernel
+// other than the default. The bitmap and hash kernels run the directed graphs, whose
+// anchors and probes the formula fixes.
+static int tc_count_part(sp_graph* g, int part, int nparts, int64_t* triangle_count) {
+  SP_TRY(ensure_symmetry(g));
+  if (!g->tc) g->tc = new TcPlan();
+  int cta_warps = g->tc_cta_warps >= 0 ? g->tc_cta_warps : tc::CTA_WARPS_DEFAULT;
+  int wu = g->tc_unroll > 0 ? g->tc_unroll : tc::WU_DEFAULT;
+  int cand = -1;
+  SP_TRY(tc_variant_pick(g, &cand));
+  if (cand >= 0) {
+    if (tc::VARIANTS[cand].bitmap) cta_warps = tc::VARIANTS[cand].cta_warps;
+    else wu = tc::VARIANTS[cand].wu;
+  }
+  g->last_variant[VAR_TC] = cand;
+  const bool dflt = g->V <= 65536 ? g->E > RANK_MIN_E && cta_warps == tc::CTA_WARPS_DEFAULT : wu == tc::WU_DEFAULT;
+  if (g->symmetric == 1 && dflt) {
+    SP_TRY(build_rank_plan(g));
+    return rank_count(g, part, nparts, triangle_count, nullptr);
+  }
+  SP_TRY(build_tc_plan(g));
+  if (nparts == 1) return tc_count(g, g->tc->order.p, g->V, cta_warps, wu, triangle_count);
+  dbuf<int32_t> mine;
+  int n = 0;
+  SP_TRY(order_part(g, part, nparts, mine, n));
+  return tc_count(g, mine.p, n, cta_warps, wu, triangle_count);
+}
+
+// Per-vertex counts of the triangles of part `part` of `nparts` into counts (device).
+static int lcc_count_part(sp_graph* g, int part, int nparts, int* counts) {
+  SP_TRY(ensure_symmetry(g));
+  if (g->symmetric == 1) {
+    SP_TRY(build_rank_plan(g));
+    return rank_count(g, part, nparts, nullptr, counts);
+  }
+  SP_TRY(build_tc_plan(g));
+  if (g->V) SP_CHECK_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * g->V, g->stream));
+  if (nparts == 1) return lcc_count(g, g->tc->order.p, g->V, counts);
+  dbuf<int32_t> mine;
+  int n = 0;
+  SP_TRY(order_part(g, part, nparts, mine, n));
+  return lcc_count(g, mine.p, n, counts);
+}
+
 }  // namespace sp
 
 extern "C" int sp_tc(sp_graph_h g, int64_t* triangle_count, int32_t variant) {
@@ -986,8 +1073,7 @@ extern "C" int sp_tc(sp_graph_h g, int64_t* triangle_count, int32_t variant) {
     set_error("sp_tc: unknown variant %d", variant);
     return SP_ERR_INVALID;
   }
-  SP_TRY(build_tc_plan(g));
-  return tc_count(g, g->tc->order.p, g->V, triangle_count);
+  return tc_count_part(g, 0, 1, triangle_count);
 }
 
 extern "C" int sp_clustering_coeff(sp_graph_h g, int32_t* cf, int32_t variant) {
@@ -1003,17 +1089,16 @@ extern "C" int sp_clustering_coeff(sp_graph_h g, int32_t* cf, int32_t variant) {
   cudaStream_t s = g->stream;
   dbuf<int> counts;
   SP_TRY(counts.alloc(g->V));
-  if (g->V) SP_CHECK_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int) * g->V, s));
   if (variant == SP_TC_PLAIN) {
     const int tb = 512;  // backend_cuda/dsl_cpp_generator.cpp:56-77
     if (g->V) {
+      SP_CHECK_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int) * g->V, s));
       tc::k_lcc_plain<<<(g->V + tb - 1) / tb, tb, 0, s>>>(g->off.p, g->adj.p, g->V, counts.p);
       SP_CHECK_LAUNCH();
     }
     return copy_out(cf, counts.p, sizeof(int32_t) * g->V, s);
   }
-  SP_TRY(build_tc_plan(g));
-  SP_TRY(lcc_count(g, g->tc->order.p, g->V, counts.p));
+  SP_TRY(lcc_count_part(g, 0, 1, counts.p));
   return copy_out(cf, counts.p, sizeof(int32_t) * g->V, s);
 }
 
@@ -1040,12 +1125,7 @@ static int check_part(const char* fn, sp_graph_h g, const void* out, int32_t par
 extern "C" int sp_tc_part(sp_graph_h g, int32_t part, int32_t nparts, int64_t* triangle_count) {
   using namespace sp;
   SP_TRY(check_part("sp_tc_part", g, triangle_count, part, nparts));
-  SP_TRY(build_tc_plan(g));
-  if (nparts == 1) return tc_count(g, g->tc->order.p, g->V, triangle_count);
-  dbuf<int32_t> mine;
-  int n = 0;
-  SP_TRY(order_part(g, part, nparts, mine, n));
-  return tc_count(g, mine.p, n, triangle_count);
+  return tc_count_part(g, part, nparts, triangle_count);
 }
 
 extern "C" int sp_clustering_coeff_part(sp_graph_h g, int32_t part, int32_t nparts, int32_t* cf) {
@@ -1054,16 +1134,7 @@ extern "C" int sp_clustering_coeff_part(sp_graph_h g, int32_t part, int32_t npar
   cudaStream_t s = g->stream;
   dbuf<int> counts;
   SP_TRY(counts.alloc(g->V));
-  if (g->V) SP_CHECK_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int) * g->V, s));
-  SP_TRY(build_tc_plan(g));
-  dbuf<int32_t> mine;
-  int n = g->V;
-  const int32_t* order = g->tc->order.p;
-  if (nparts > 1) {
-    SP_TRY(order_part(g, part, nparts, mine, n));
-    order = mine.p;
-  }
-  SP_TRY(lcc_count(g, order, n, counts.p));
+  SP_TRY(lcc_count_part(g, part, nparts, counts.p));
   return copy_out(cf, counts.p, sizeof(int32_t) * g->V, s);
 }
 
@@ -1205,8 +1276,7 @@ extern "C" int sp_tc_dynamic(sp_graph_h g, int64_t n, const char* type, const in
     *triangle_count += dcount;
     return SP_OK;
   }
-  SP_TRY(build_tc_plan(g));
-  return tc_count(g, g->tc->order.p, g->V, triangle_count);
+  return tc_count_part(g, 0, 1, triangle_count);
 }
 
 // DynCF's Batch block (dynamicDSLCodes/dynamicBatchClustering:44-53): the batch, then
@@ -1239,8 +1309,6 @@ extern "C" int sp_clustering_coeff_dynamic(sp_graph_h g, int64_t n, const char* 
     SP_CHECK_LAUNCH();
     return copy_out(cf, x.p, sizeof(int32_t) * g->V, s);
   }
-  SP_CHECK_CUDA(cudaMemsetAsync(delta.p, 0, sizeof(int) * g->V, s));
-  SP_TRY(build_tc_plan(g));
-  SP_TRY(lcc_count(g, g->tc->order.p, g->V, delta.p));
+  SP_TRY(lcc_count_part(g, 0, 1, delta.p));
   return copy_out(cf, delta.p, sizeof(int32_t) * g->V, s);
 }
