@@ -10,28 +10,22 @@
 // so the source is excluded; no halving — the manual CUDA BC bcManualv5.cu:104
 // halves, the generated code does not).
 //
-// B200 design — multi-source traversal (many sources share one pass over the edges):
-//  * up to 32*NW sources per batch; per vertex a 64-bit mask says for which sources
-//    of the batch it sits in the current frontier; sigma[v][b] (FP64, exact path
-//    counts below 2^53) and delta[v][b] (FP32) are vertex-major, so the per-source
-//    updates of one edge are coalesced across the warp's lanes;
-//  * forward level d: lanes walk a frontier vertex's edges; q = mask & ~seen[w] are
-//    the sources that reach w first at level d+1; atomicOr marks them, the first
-//    marker appends w to the level list, then lanes (one per source bit) add
-//    sigma with FP64 atomics (integer-valued, so the sum is exact in any order);
-//  * backward level d: the masks of level d+1 are scattered into a dense array; for
-//    each (v, mask) of level d the lanes pull q[w][b] = (1 + delta[w][b]) / sigma[w][b]
-//    of the successors in edge order (stored in FP64 when w's dependency became final),
-//    the loads of BU successors in flight together, and delta[v][b] = sigma[v][b] *
-//    sum q — one 8-byte load and one add per successor instead of two loads and an FP64
-//    division; no atomics, deterministic;
-//  * level-list entries of vertices with more than hub_deg edges (default 64) are cut
-//    into hub_chunk-edge pieces (default 64) that all warps share (one extra barrier
-//    per level); their backward partials meet in an FP64 scratch through atomics;
-//  * BC accumulates per vertex over the batch's sources in source order (FP64).
-// One cooperative launch runs every batch of a graph (bounded grid barriers); the
-// many-small-graphs form runs one CTA per graph in a persistent launch with a
-// work queue (largest graphs first) and block-level barriers.
+// Two forms, both multi-source (many sources share one pass over the edges; per vertex, a
+// 64-bit mask says for which sources of the batch it sits in a level):
+//  * the gather form (sp_bc_gather.cuh), the default: path counts and dependencies are both
+//    summed by the entry that needs them, one row of doubles per vertex;
+//  * the push / pull form here, for a forward direction chosen per level (knob bc.dir, or a
+//    loaded level model). Forward push: q = mask & ~seen[w] are the sources that reach w
+//    first at level d+1; atomicOr marks them, the first marker appends w to the level list,
+//    then lanes (one per source bit) add sigma with FP64 atomics (integer-valued, so the
+//    sum is exact in any order). Backward level d: for each (v, mask) the lanes sum
+//    q[w][b] = (1 + delta[w][b]) / sigma[w][b] of the successors in edge order, BU
+//    successors' loads in flight; BC accumulates over the batch's sources in source order.
+// In both, level-list entries of vertices with more than hub_deg edges (default 64) are cut
+// into hub_chunk-edge pieces (default 64) that all warps share, and one cooperative launch
+// runs every batch (bounded grid barriers). Many graphs run as one graph in the gather form,
+// or (knob bc.cluster, or when that does not fit) one CTA or cluster per graph from a work
+// queue, largest first.
 #include <cooperative_groups.h>
 
 #include <climits>
@@ -40,6 +34,8 @@
 #include "sp_internal.cuh"
 #include "sp_mlp_dev.cuh"
 #include "sp_sync.cuh"
+
+#include "sp_bc_gather.cuh"
 
 namespace sp {
 
@@ -62,10 +58,7 @@ constexpr int CLUSTER_DEFAULT = 1;  // CTAs per graph in the many-graphs form (b
 // registers (3 CTAs per SM), 121 ms with 4 at 128 registers; 1000 ER graphs: 135 ->
 // 104 ms.
 constexpr int BU = 2;
-// The same for the many-graphs kernels: with one q load per successor, 1000 ER graphs
-// take 92.8 ms at 4 in flight, 126.6 ms at 2 (which spills in k_bc_graphs<1>) and
-// 103.4 ms before q; R-MAT 20 (grid kernel, BU) 74.1 ms at 2, 76.7 at 4.
-constexpr int BU_GRAPHS = 4;
+constexpr double UNION_BYTES = 32e9;  // most rows and scratch of the many-graphs form as one graph
 // 32-edge chunks of one entry whose loads and atomics are in flight together in the
 // forward sweep.
 constexpr int FU = 2;
@@ -768,21 +761,56 @@ __global__ void __launch_bounds__(GRID_THREADS, 4) k_bc_grid(GridArgs a) {
   }
 }
 
-// ---- many small graphs: one CTA per graph, persistent, work queue
+// ---- the gather form (sp_bc_gather.cuh) on one graph: one cooperative launch, all batches
+struct GatherArgs {
+  Gather G;
+  const int32_t* srcs;
+  const int32_t* cols;  // column of each source (null: its place in its batch)
+  const int32_t* boff;  // [batches + 1] first source of each batch (null: k * batch)
+  int nsrc;
+  int batch;  // sources per batch
+  int batches;
+  GridBar* bar;
+  int32_t* lvl_out;
+  double* sig_out;
+};
+
+template <int SW>
+__global__ void __launch_bounds__(GRID_THREADS, 4) k_bc_gather(GatherArgs a) {
+  extern __shared__ Picked s_pick[];
+  __shared__ Gather s_g;
+  if (threadIdx.x == 0) s_g = a.G;
+  __syncthreads();
+  GridSync gs{a.bar};
+  for (int k = 0; k < a.batches; ++k) {
+    const int s0 = a.boff ? a.boff[k] : k * a.batch;
+    const int n = a.boff ? a.boff[k + 1] - s0 : min(a.batch, a.nsrc - s0);
+    if (!gather_batch<SW>(s_g, a.srcs + s0, a.cols ? a.cols + s0 : nullptr, n, gs, s_pick[threadIdx.x >> 5],
+                              a.lvl_out, a.sig_out)) {
+      if (threadIdx.x == 0 && a.bar->error) atomicCAS(a.G.err, 0, 3);
+      return;
+    }
+  }
+}
+
+// ---- many small graphs: one team (a CTA, or a cluster of C CTAs) per graph, persistent,
+// work queue, largest graphs first
 struct GraphsArgs {
   const int32_t* off;     // union CSR rows
   const int32_t* adj;     // union CSR neighbours (global ids)
+  const int32_t* roff;    // in-edges (the same arrays when sym)
+  const int32_t* radj;
+  int sym;
   const int32_t* voff;    // [G+1] vertex ranges
   const int32_t* soff;    // [G+1] source ranges
   const int32_t* srcs;    // global source ids
   const int32_t* order;   // graphs, largest first
   int G;
   int* next;              // work-queue counter
-  // per-CTA scratch (sized for the largest graph)
-  double* sigma;
-  float* delta;
-  double* q;
-  unsigned long long* masks;  // 3 * vmax per CTA
+  // per-team scratch (sized for the largest graph)
+  double* row;
+  unsigned long long* masks;  // mwords per team
+  size_t mwords;              // >= 6 * vmax, a multiple of 4 (32-byte records)
   int32_t* flv;
   unsigned long long* flm;
   int* lo;
@@ -792,112 +820,95 @@ struct GraphsArgs {
   int* err;
 };
 
-template <int NW>
-__global__ void __launch_bounds__(CTA_THREADS) k_bc_graphs(GraphsArgs a) {
-  constexpr int SW = 32 * NW;
-  __shared__ int s_g;
-  __shared__ int32_t s_src[SW];
-  BlockSync bs;
-  const int slot = blockIdx.x;
-  Work W;
-  W.sigma = a.sigma + (size_t)slot * a.vmax * SW;
-  W.delta = a.delta + (size_t)slot * a.vmax * SW;
-  W.q = a.q + (size_t)slot * a.vmax * SW;
-  W.seen = a.masks + (size_t)slot * a.vmax * 3;
-  W.nxt = W.seen + a.vmax;
-  W.dense = W.nxt + a.vmax;
-  W.flv = a.flv + (size_t)slot * a.cap;
-  W.flm = a.flm + (size_t)slot * a.cap;
-  W.cap = a.cap;
-  W.lo = a.lo + (size_t)slot * (a.maxd + 2);
-  W.maxd = a.maxd;
-  W.cnt = a.cnt + slot;
-  W.err = a.err;
-  W.off = a.off;
-  W.adj = a.adj;
-  W.hub_cap = 0;
-  W.hub_deg = bc::HUB_DEG;
-  W.hub_chunk = bc::HUB_CHUNK;
-  W.hub_ent = W.hub_base = nullptr;
-  W.hub_cnt = nullptr;
-  W.dacc = nullptr;
+// The graphs of one team, slot `slot`; k(): the next queue position, the same for all of
+// the team, and free to be overwritten when it returns. W: this CTA's arguments, in shared
+// memory.
+template <int SW, class S, class K>
+__device__ __forceinline__ void run_graphs(const GraphsArgs& a, int slot, S& sync, K&& next, Picked& pk,
+                                           int32_t* s_src, Gather& W) {
+  if (threadIdx.x == 0) {
+    W.row = a.row + (size_t)slot * a.vmax * SW;
+    W.dacc = nullptr;
+    W.mask = (Masks*)(a.masks + (size_t)slot * a.mwords);
+    W.back = (unsigned long long*)(W.mask + a.vmax);
+    W.bstride = a.vmax;
+    W.flv = a.flv + (size_t)slot * a.cap;
+    W.flm = a.flm + (size_t)slot * a.cap;
+    W.cap = a.cap;
+    W.lo = a.lo + (size_t)slot * (a.maxd + 2);
+    W.maxd = a.maxd;
+    W.cnt = a.cnt + slot;
+    W.err = a.err;
+    W.adj = a.adj;
+    W.radj = a.radj;
+    W.sym = a.sym;
+    W.pcap = W.hcap = 0;  // rows are not split: a team works on one graph
+    W.hub_deg = W.hub_chunk = 0;
+    W.piece = W.rpiece = nullptr;
+    W.hub = W.rhub = nullptr;
+    W.plo = W.hlo = W.pc = nullptr;
+  }
+  __syncthreads();
+  const int gt = sync.tid(), nt = sync.nthreads();
+  for (size_t i = gt; i < a.mwords; i += nt) ((unsigned long long*)W.mask)[i] = 0ull;  // as after a batch
   while (true) {
-    if (threadIdx.x == 0) s_g = atomicAdd(a.next, 1);
-    __syncthreads();
-    const int k = s_g;
-    __syncthreads();
+    const int k = next();
     if (k >= a.G) break;
     const int g = a.order[k];
     const int vb = a.voff[g], n = a.voff[g + 1] - vb;
-    W.off = a.off + vb;
-    W.vbase = vb;
-    W.V = n;
-    W.bc = a.bc + vb;
+    if (threadIdx.x == 0) {
+      W.off = a.off + vb;
+      W.roff = a.roff + vb;
+      W.vbase = vb;
+      W.V = n;
+      W.bc = a.bc + vb;
+    }
     const int sb = a.soff[g], ns = a.soff[g + 1] - sb;
     for (int s0 = 0; s0 < ns; s0 += SW) {
       const int nb = min(SW, ns - s0);
+      // every CTA keeps its own copy
       for (int t = threadIdx.x; t < nb; t += blockDim.x) s_src[t] = a.srcs[sb + s0 + t] - vb;
       __syncthreads();
-      if (!run_batch_any<NW, BU_GRAPHS>(W, s_src, nb, bs)) return;
+      if (!gather_batch<SW>(W, s_src, nullptr, nb, sync, pk)) return;
     }
   }
+}
+
+template <int SW>
+__global__ void __launch_bounds__(CTA_THREADS, 2) k_bc_graphs(GraphsArgs a) {
+  __shared__ int s_g;
+  __shared__ int32_t s_src[SW];
+  extern __shared__ Picked s_pick[];
+  __shared__ Gather s_w;
+  BlockSync bs;
+  auto next = [&]() {
+    __syncthreads();
+    if (threadIdx.x == 0) s_g = atomicAdd(a.next, 1);
+    __syncthreads();
+    return s_g;
+  };
+  run_graphs<SW>(a, blockIdx.x, bs, next, s_pick[threadIdx.x >> 5], s_src, s_w);
 }
 
 // The many-graphs form with a cluster of C CTAs per graph (C > 1): the work queue hands
 // graphs to clusters, largest first, and each graph's batches run with cluster barriers,
 // so a large graph gets C SMs' worth of warps instead of one CTA's.
-template <int NW, int C>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(CTA_THREADS) k_bc_clusters(GraphsArgs a) {
-  constexpr int SW = 32 * NW;
+template <int SW, int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(CTA_THREADS, 2) k_bc_clusters(GraphsArgs a) {
   __shared__ int s_g;
   __shared__ int32_t s_src[SW];
+  extern __shared__ Picked s_pick[];
+  __shared__ Gather s_w;
   cg::cluster_group cl = cg::this_cluster();
   ClusterSync cs;
-  const int slot = blockIdx.x / C;
-  const bool leader = cl.block_rank() == 0;
-  Work W;
-  W.sigma = a.sigma + (size_t)slot * a.vmax * SW;
-  W.delta = a.delta + (size_t)slot * a.vmax * SW;
-  W.q = a.q + (size_t)slot * a.vmax * SW;
-  W.seen = a.masks + (size_t)slot * a.vmax * 3;
-  W.nxt = W.seen + a.vmax;
-  W.dense = W.nxt + a.vmax;
-  W.flv = a.flv + (size_t)slot * a.cap;
-  W.flm = a.flm + (size_t)slot * a.cap;
-  W.cap = a.cap;
-  W.lo = a.lo + (size_t)slot * (a.maxd + 2);
-  W.maxd = a.maxd;
-  W.cnt = a.cnt + slot;
-  W.err = a.err;
-  W.off = a.off;
-  W.adj = a.adj;
-  W.hub_cap = 0;
-  W.hub_deg = HUB_DEG;
-  W.hub_chunk = HUB_CHUNK;
-  W.hub_ent = W.hub_base = nullptr;
-  W.hub_cnt = nullptr;
-  W.dacc = nullptr;
-  while (true) {
-    if (leader && threadIdx.x == 0) s_g = atomicAdd(a.next, 1);
+  auto next = [&]() {
+    if (cl.block_rank() == 0 && threadIdx.x == 0) s_g = atomicAdd(a.next, 1);
     cl.sync();
     const int k = *cl.map_shared_rank(&s_g, 0);
     cl.sync();  // every CTA has read the leader's s_g before it is overwritten
-    if (k >= a.G) break;
-    const int g = a.order[k];
-    const int vb = a.voff[g], n = a.voff[g + 1] - vb;
-    W.off = a.off + vb;
-    W.vbase = vb;
-    W.V = n;
-    W.bc = a.bc + vb;
-    const int sb = a.soff[g], ns = a.soff[g + 1] - sb;
-    for (int s0 = 0; s0 < ns; s0 += SW) {
-      const int nb = min(SW, ns - s0);
-      // every CTA keeps its own copy: run_batch reads srcs from the caller's CTA
-      for (int t = threadIdx.x; t < nb; t += blockDim.x) s_src[t] = a.srcs[sb + s0 + t] - vb;
-      __syncthreads();
-      if (!run_batch_any<NW, BU_GRAPHS>(W, s_src, nb, cs)) return;
-    }
-  }
+    return k;
+  };
+  run_graphs<SW>(a, blockIdx.x / C, cs, next, s_pick[threadIdx.x >> 5], s_src, s_w);
 }
 
 __global__ void k_stamp_time(unsigned long long* t) {
@@ -909,6 +920,20 @@ __global__ void k_stamp_time(unsigned long long* t) {
 __global__ void k_zero(void* p, size_t words) {
   unsigned long long* q = (unsigned long long*)p;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x) q[i] = 0ull;
+}
+
+// What a call of the gather form starts from: zeros (in 16-byte words).
+__global__ void __launch_bounds__(256) k_clear(double2* dacc, size_t nd, double2* masks, size_t nm, double2* bc,
+                                               size_t nb, GridBar* bar, int* err) {
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = t; i < nd; i += nt) dacc[i] = make_double2(0.0, 0.0);
+  for (size_t i = t; i < nm; i += nt) masks[i] = make_double2(0.0, 0.0);
+  for (size_t i = t; i < nb; i += nt) bc[i] = make_double2(0.0, 0.0);
+  if (t == 0) {
+    bar->arrived = 0;
+    bar->error = 0;
+    *err = 0;
+  }
 }
 
 __global__ void k_to_float(const double* __restrict__ a, float* __restrict__ b, int n) {
@@ -976,6 +1001,9 @@ struct BcPlan {
   dbuf<int32_t> flv, lo, cnt, srcs, level, aux;
   dbuf<GridBar> bar;
   dbuf<int> err;
+  // gather form: the pieces and split entries of the level lists
+  dbuf<int4> piece, rpiece;
+  dbuf<int32_t> hub, rhub, plo;
   // learned variant inputs (vstat < 0: not yet) and the choice for var_nsrc sources
   int vstat = -1;
   int64_t vmax = 0, vsq = 0, vrows[4] = {}, vedges[4] = {};
@@ -1075,8 +1103,147 @@ static int bc_variant_pick(sp_graph* g, int nsrc, int* cand) {
   return SP_OK;
 }
 
+// bc.hub_deg / bc.hub_chunk of a call: the knobs, the learned variant, or the defaults.
+static int bc_split(sp_graph* g, int nsrc, int* hub_deg, int* hub_chunk) {
+  *hub_deg = g->bc_hub_deg > 0 ? g->bc_hub_deg : bc::HUB_DEG;
+  *hub_chunk = g->bc_hub_chunk > 0 ? g->bc_hub_chunk : bc::HUB_CHUNK;
+  int cand = -1;
+  SP_TRY(bc_variant_pick(g, nsrc, &cand));
+  if (cand >= 0) {
+    *hub_deg = bc::VARIANTS[cand].hub_deg;
+    *hub_chunk = bc::VARIANTS[cand].hub_chunk;
+  }
+  g->last_variant[VAR_BC] = cand;
+  return SP_OK;
+}
+
+static int bc_status(sp_graph* g, int maxd) {
+  int herr = 0;
+  SP_TRY(copy_out(&herr, g->bc->err.p, sizeof(int), g->stream));
+  if (!herr) return SP_OK;
+  set_error("sp_bc: device error %d (1 level lists full, 2 deeper than %d levels, 3 barrier timeout)", herr, maxd);
+  return herr == 3 ? SP_ERR_TIMEOUT : SP_ERR_UNSUPPORTED;
+}
+
+// The gather form over all batches of a call: sources d_srcs[0 .. nsrc), batch of them at a
+// time, column k for the k-th of a batch; or (d_cols) batches d_boff[k] .. d_boff[k + 1] with
+// given columns below `width`. A graph is listed in at most maxd levels.
+static int bc_gather(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch, int width, int maxd, int32_t* lvl_out,
+                     double* sig_out, const int32_t* d_cols = nullptr, const int32_t* d_boff = nullptr,
+                     int batches = 0) {
+  SP_TRY(ensure_symmetry(g));  // sums run over in-edges
+  BcPlan* p = g->bc;
+  cudaStream_t s = g->stream;
+  const int V = g->V;
+  const int SW = width > 32 ? 64 : width > 16 ? 32 : 16;
+  const size_t cap = (size_t)V * std::min(width, 16) + 1024;  // level-list entries (vertex, mask)
+  bc::GatherArgs a;
+  bc::Gather& W = a.G;
+  SP_TRY(bc_split(g, nsrc, &W.hub_deg, &W.hub_chunk));
+  // Pieces of one pass over the graph: at most E / chunk + E / hub_deg. A vertex is listed
+  // once per level it is in; four levels of it fit, or all 16 for up to 16 sources (what
+  // the caller falls back to).
+  const double E = (double)g->E;
+  while (16 * (E / W.hub_chunk + E / W.hub_deg) > (double)(1 << 30)) {  // counts stay below 2^31
+    W.hub_deg *= 2;
+    W.hub_chunk *= 2;
+  }
+  const double copies = width > 16 ? 4 : width;
+  const size_t pcap = (size_t)(copies * (E / W.hub_chunk + E / W.hub_deg)) + 1024;
+  const size_t hcap = (size_t)(copies * (E / W.hub_deg)) + 1024;
+  SP_TRY(p->sigma.alloc((size_t)V * SW));
+  SP_TRY(p->dacc.alloc((size_t)V * SW));
+  SP_TRY(p->masks.alloc((size_t)V * 6));
+  SP_TRY(p->flv.alloc(cap));
+  SP_TRY(p->flm.alloc(cap));
+  SP_TRY(p->lo.alloc(maxd + 2));
+  SP_TRY(p->plo.alloc(2 * (size_t)(maxd + 2) + 6));
+  SP_TRY(p->cnt.alloc(1));
+  SP_TRY(p->bc.alloc(V));
+  SP_TRY(p->bar.alloc(1));
+  SP_TRY(p->err.alloc(1));
+  SP_TRY(p->piece.alloc(pcap));
+  SP_TRY(p->hub.alloc(hcap));
+  const bool sym = g->symmetric == 1;
+  if (!sym) {
+    SP_TRY(p->rpiece.alloc(2 * pcap));
+    SP_TRY(p->rhub.alloc(2 * hcap));
+  }
+  // (an odd count's last double lies before the buffer's 16 spare bytes)
+  bc::k_clear<<<num_sms() * 8, 256, 0, s>>>((double2*)p->dacc.p, (size_t)V * SW / 2, (double2*)p->masks.p,
+                                            (size_t)V * 3, (double2*)p->bc.p, ((size_t)V + 1) / 2, p->bar.p,
+                                            p->err.p);
+  SP_CHECK_LAUNCH();
+  W.off = g->off.p;
+  W.adj = g->adj.p;
+  W.roff = sym ? g->off.p : g->roff.p;
+  W.radj = sym ? g->adj.p : g->radj.p;
+  W.sym = sym ? 1 : 0;
+  W.vbase = 0;
+  W.V = V;
+  W.row = p->sigma.p;
+  W.dacc = p->dacc.p;
+  W.mask = (bc::Masks*)p->masks.p;
+  W.back = p->masks.p + 4 * (size_t)V;
+  W.bstride = V;
+  W.flv = p->flv.p;
+  W.flm = p->flm.p;
+  W.cap = (int)std::min<size_t>(cap, INT_MAX);
+  W.lo = p->lo.p;
+  W.maxd = maxd;
+  W.cnt = p->cnt.p;
+  W.bc = p->bc.p;
+  W.err = p->err.p;
+  W.pcap = (int)pcap;
+  W.hcap = (int)hcap;
+  W.piece = p->piece.p;
+  W.hub = p->hub.p;
+  W.plo = p->plo.p;
+  W.hlo = p->plo.p + maxd + 2;
+  W.pc = p->plo.p + 2 * (maxd + 2);
+  W.rpiece = sym ? nullptr : p->rpiece.p;
+  W.rhub = sym ? nullptr : p->rhub.p;
+  a.srcs = d_srcs;
+  a.cols = d_cols;
+  a.boff = d_boff;
+  a.nsrc = nsrc;
+  a.batch = batch;
+  a.batches = d_boff ? batches : (nsrc + batch - 1) / batch;
+  a.bar = p->bar.p;
+  a.lvl_out = lvl_out;
+  a.sig_out = sig_out;
+  p->trace_n = 0;
+  void* params[] = {&a};
+  int per_sm = 0;
+  const void* fn = SW == 64   ? (const void*)bc::k_bc_gather<64>
+                   : SW == 32 ? (const void*)bc::k_bc_gather<32>
+                              : (const void*)bc::k_bc_gather<16>;
+  constexpr int smem = (int)(sizeof(bc::Picked) * (bc::GRID_THREADS / 32));
+  SP_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SP_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bc::GRID_THREADS, smem));
+  // a warp for every few items of the widest level a graph can have, so that a small graph's
+  // barriers wait for few CTAs
+  const double items = (double)V * SW / 128 + E / W.hub_chunk;
+  const int fit = num_sms() * std::max(1, std::min(per_sm, 4));
+  const int grid = (int)std::min<double>(fit, std::max<double>(num_sms() / 2, items / (bc::GRID_THREADS / 32)));
+  SP_CHECK_CUDA(cudaLaunchCooperativeKernel(fn, grid, bc::GRID_THREADS, params, smem, s));
+  g_launches++;
+  return bc_status(g, maxd);
+}
+
+// The push / pull form, whose forward direction per level is chosen by the knob bc.dir or
+// the level model; bc.dir = 0 (the default without a model) takes the gather form.
 static int bc_grid(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch_hint, int32_t* lvl_out = nullptr,
                    double* sig_out = nullptr) {
+  {
+    std::vector<float> packed;
+    const unsigned lgen = mlp_level_model(packed);
+    if ((g->bc_dir >= 0 ? g->bc_dir : (lgen ? 4 : bc::DIR_DEFAULT)) == 0)
+    {
+      const int batch = std::max(1, std::min(std::min(batch_hint, 64), nsrc));
+      return bc_gather(g, d_srcs, nsrc, batch, batch, 1 << 14, lvl_out, sig_out);
+    }
+  }
   BcPlan* p = g->bc;
   cudaStream_t s = g->stream;
   const int V = g->V;
@@ -1136,17 +1303,7 @@ static int bc_grid(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch_hint,
   W.hub_base = p->hub_base.p;
   W.hub_cnt = p->hub_cnt.p;
   W.hub_cap = hub_cap;
-  W.hub_deg = g->bc_hub_deg > 0 ? g->bc_hub_deg : bc::HUB_DEG;
-  W.hub_chunk = g->bc_hub_chunk > 0 ? g->bc_hub_chunk : bc::HUB_CHUNK;
-  {
-    int cand = -1;
-    SP_TRY(bc_variant_pick(g, nsrc, &cand));
-    if (cand >= 0) {
-      W.hub_deg = bc::VARIANTS[cand].hub_deg;
-      W.hub_chunk = bc::VARIANTS[cand].hub_chunk;
-    }
-    g->last_variant[VAR_BC] = cand;
-  }
+  SP_TRY(bc_split(g, nsrc, &W.hub_deg, &W.hub_chunk));
   W.dacc = p->dacc.p;
   // forward direction per level
   std::vector<float> packed;
@@ -1230,12 +1387,7 @@ static int bc_grid(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch_hint,
   const int grid = num_sms() * std::max(1, std::min(per_sm, 4));
   SP_CHECK_CUDA(cudaLaunchCooperativeKernel(fn, grid, bc::GRID_THREADS, params, 0, s));
   g_launches++;
-  int herr = 0;
-  SP_TRY(copy_out(&herr, p->err.p, sizeof(int), s));
-  if (herr) {
-    set_error("sp_bc: device error %d (1 level lists full, 2 deeper than %d levels, 3 barrier timeout)", herr, maxd);
-    return herr == 3 ? SP_ERR_TIMEOUT : SP_ERR_UNSUPPORTED;
-  }
+  SP_TRY(bc_status(g, maxd));
   if (W.trace) {  // the end of the last traced level
     int n = 0;
     SP_TRY(copy_out(&n, p->tcount.p, sizeof(int), s));
@@ -1314,13 +1466,19 @@ extern "C" int sp_bc(sp_graph_h g, const int32_t* sources, int32_t nsrc, float* 
     bc::k_to_float<<<num_sms() * 4, 256, 0, s>>>(p->bc.p, p->fout.p, g->V);
     SP_CHECK_LAUNCH();
   } else if (variant == SP_BC_BATCHED) {
-    SP_TRY(p->srcs.alloc(nsrc));
+    SP_TRY(p->srcs.alloc(2 * (size_t)nsrc));
     SP_CHECK_CUDA(cudaMemcpyAsync(p->srcs.p, hs.data(), sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, s));
     const int batch = g->bc_batch > 0 ? (int)g->bc_batch : 64;
-    int st = bc_grid(g, p->srcs.p, nsrc, batch);
+    int32_t* srcs = p->srcs.p;
+    if (nsrc > 1 && nsrc <= bc::ORDER_MAX) {
+      srcs = p->srcs.p + nsrc;
+      bc::k_order_sources<<<(nsrc + 255) / 256, 256, 0, s>>>(g->off.p, p->srcs.p, nsrc, srcs);
+      SP_CHECK_LAUNCH();
+    }
+    int st = bc_grid(g, srcs, nsrc, batch);
     // level lists hold at most V * min(batch, 16) entries; a deep graph can need more
     // when many sources share a batch, so retry with 16 sources per batch (always fits)
-    if (st == SP_ERR_UNSUPPORTED && batch > 16) st = bc_grid(g, p->srcs.p, nsrc, 16);
+    if (st == SP_ERR_UNSUPPORTED && batch > 16) st = bc_grid(g, srcs, nsrc, 16);
     SP_TRY(st);
     bc::k_to_float<<<num_sms() * 4, 256, 0, s>>>(p->bc.p, p->fout.p, g->V);
     SP_CHECK_LAUNCH();
@@ -1330,6 +1488,116 @@ extern "C" int sp_bc(sp_graph_h g, const int32_t* sources, int32_t nsrc, float* 
   }
   return copy_out(BC, p->fout.p, sizeof(float) * g->V, s);
 }
+
+namespace sp {
+// Many graphs, a team (a CTA, or a cluster of bc.cluster CTAs) each, SW sources at a time;
+// 16 if the level lists of more do not fit (16 always fit).
+static int bc_graph_teams(sp_graph* g, int ngraphs, const std::vector<int32_t>& voff, const std::vector<int32_t>& soff,
+                          const std::vector<int32_t>& hs, int vmax, int smax, int SW, float* BC) {
+  BcPlan* p = g->bc;
+  cudaStream_t s = g->stream;
+  const int maxd = 4096;
+  const int nsrc = soff[ngraphs];
+  const bool sym = g->symmetric == 1;
+  // graphs the teams take from the queue, largest first
+  std::vector<int32_t> order(ngraphs);
+  for (int k = 0; k < ngraphs; ++k) order[k] = k;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return (int64_t)(voff[a + 1] - voff[a]) * (soff[a + 1] - soff[a]) > (int64_t)(voff[b + 1] - voff[b]) * (soff[b + 1] - soff[b]);
+  });
+  const int cap = vmax * std::min(std::max(1, std::min(smax, SW)), 16) + 1024;
+  int per_sm = 0;
+  const void* fn = SW == 64   ? (const void*)bc::k_bc_graphs<64>
+                   : SW == 32 ? (const void*)bc::k_bc_graphs<32>
+                              : (const void*)bc::k_bc_graphs<16>;
+  constexpr int smem = (int)(sizeof(bc::Picked) * (bc::CTA_THREADS / 32));
+  SP_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SP_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bc::CTA_THREADS, smem));
+  const int C = g->bc_cluster > 0 ? g->bc_cluster : bc::CLUSTER_DEFAULT;
+  // one scratch slot per team (a CTA, or a cluster of C CTAs)
+  const int teams = std::max(1, std::min(num_sms() * std::max(1, std::min(per_sm, 2)) / C, ngraphs));
+  const int ctas = teams;
+  SP_TRY(p->sigma.alloc((size_t)ctas * vmax * SW));
+  const size_t mwords = ((size_t)vmax * 6 + 3) & ~(size_t)3;
+  SP_TRY(p->masks.alloc(ctas * mwords));
+  SP_TRY(p->flv.alloc((size_t)ctas * cap));
+  SP_TRY(p->flm.alloc((size_t)ctas * cap));
+  SP_TRY(p->lo.alloc((size_t)ctas * (maxd + 2)));
+  SP_TRY(p->cnt.alloc(ctas + 1));
+  SP_TRY(p->bc.alloc(g->V));
+  SP_TRY(p->srcs.alloc(std::max(1, nsrc) + 2 * (ngraphs + 1) + ngraphs));
+  SP_TRY(p->err.alloc(1));
+  SP_TRY(p->fout.alloc(g->V));
+  int32_t* d_srcs = p->srcs.p;
+  int32_t* d_voff = d_srcs + std::max(1, nsrc);
+  int32_t* d_soff = d_voff + ngraphs + 1;
+  int32_t* d_order = d_soff + ngraphs + 1;
+  if (nsrc) SP_CHECK_CUDA(cudaMemcpyAsync(d_srcs, hs.data(), sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, s));
+  SP_CHECK_CUDA(cudaMemcpyAsync(d_voff, voff.data(), sizeof(int32_t) * (ngraphs + 1), cudaMemcpyHostToDevice, s));
+  SP_CHECK_CUDA(cudaMemcpyAsync(d_soff, soff.data(), sizeof(int32_t) * (ngraphs + 1), cudaMemcpyHostToDevice, s));
+  SP_CHECK_CUDA(cudaMemcpyAsync(d_order, order.data(), sizeof(int32_t) * ngraphs, cudaMemcpyHostToDevice, s));
+  bc::k_zero<<<num_sms() * 8, 256, 0, s>>>(p->bc.p, (size_t)g->V);
+  g_launches++;
+  SP_CHECK_CUDA(cudaMemsetAsync(p->cnt.p, 0, sizeof(int) * (ctas + 1), s));
+  SP_CHECK_CUDA(cudaMemsetAsync(p->err.p, 0, sizeof(int), s));
+  bc::GraphsArgs a;
+  a.off = g->off.p;
+  a.adj = g->adj.p;
+  a.roff = sym ? g->off.p : g->roff.p;
+  a.radj = sym ? g->adj.p : g->radj.p;
+  a.sym = sym ? 1 : 0;
+  a.voff = d_voff;
+  a.soff = d_soff;
+  a.srcs = d_srcs;
+  a.order = d_order;
+  a.G = ngraphs;
+  a.next = p->cnt.p + ctas;
+  a.row = p->sigma.p;
+  a.masks = p->masks.p;
+  a.mwords = mwords;
+  a.flv = p->flv.p;
+  a.flm = p->flm.p;
+  a.lo = p->lo.p;
+  a.cnt = p->cnt.p;
+  a.bc = p->bc.p;
+  a.vmax = vmax;
+  a.cap = cap;
+  a.maxd = maxd;
+  a.err = p->err.p;
+  if (C == 1) {
+    void* params[] = {&a};
+    SP_CHECK_CUDA(cudaLaunchKernel(fn, teams, bc::CTA_THREADS, params, smem, s));
+  } else {
+#define SP_BC_CLUSTERS(CC)                                                                 \
+  {                                                                                        \
+    auto k = SW == 64   ? bc::k_bc_clusters<64, CC>                                        \
+             : SW == 32 ? bc::k_bc_clusters<32, CC>                                        \
+                        : bc::k_bc_clusters<16, CC>;                                       \
+    SP_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
+    k<<<teams * C, bc::CTA_THREADS, smem, s>>>(a);                                         \
+  }
+    if (C == 2) {
+      SP_BC_CLUSTERS(2)
+    } else if (C == 4) {
+      SP_BC_CLUSTERS(4)
+    } else {
+      SP_BC_CLUSTERS(8)
+    }
+#undef SP_BC_CLUSTERS
+  }
+  SP_CHECK_LAUNCH();
+  int herr = 0;
+  SP_TRY(copy_out(&herr, p->err.p, sizeof(int), s));
+  if (herr == 1 && SW > 16) return bc_graph_teams(g, ngraphs, voff, soff, hs, vmax, smax, 16, BC);
+  if (herr) {
+    set_error("sp_bc_graphs: device error %d (1 level lists full, 2 deeper than %d levels)", herr, maxd);
+    return SP_ERR_UNSUPPORTED;
+  }
+  bc::k_to_float<<<num_sms() * 4, 256, 0, s>>>(p->bc.p, p->fout.p, g->V);
+  SP_CHECK_LAUNCH();
+  return copy_out(BC, p->fout.p, sizeof(float) * g->V, s);
+}
+}  // namespace sp
 
 extern "C" int sp_bc_graphs(sp_graph_h g, int32_t ngraphs, const int32_t* vertex_offset, const int32_t* source_offset,
                             const int32_t* sources, float* BC) {
@@ -1369,104 +1637,48 @@ extern "C" int sp_bc_graphs(sp_graph_h g, int32_t ngraphs, const int32_t* vertex
       return SP_ERR_INVALID;
     }
   }
-  // graphs the CTAs take from the queue, largest first
-  std::vector<int32_t> order(ngraphs);
-  for (int k = 0; k < ngraphs; ++k) order[k] = k;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-    return (int64_t)(voff[a + 1] - voff[a]) * (soff[a + 1] - soff[a]) > (int64_t)(voff[b + 1] - voff[b]) * (soff[b + 1] - soff[b]);
-  });
-  const int NW = smax > 32 ? 2 : 1;
-  const int SW = 32 * NW;
+  SP_TRY(ensure_symmetry(g));  // sums run over in-edges
   const int maxd = 4096;
-  const int cap = vmax * std::min(std::max(1, std::min(smax, SW)), 16) + 1024;
-  int per_sm = 0;
-  const void* fn = NW == 2 ? (const void*)bc::k_bc_graphs<2> : (const void*)bc::k_bc_graphs<1>;
-  SP_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bc::CTA_THREADS, 0));
-  const int C = g->bc_cluster > 0 ? g->bc_cluster : bc::CLUSTER_DEFAULT;
-  // one scratch slot per team (a CTA, or a cluster of C CTAs)
-  const int teams = std::max(1, std::min(num_sms() * std::max(1, std::min(per_sm, 2)) / C, ngraphs));
-  const int ctas = teams;
-  SP_TRY(p->sigma.alloc((size_t)ctas * vmax * SW));
-  SP_TRY(p->delta.alloc((size_t)ctas * vmax * SW));
-  SP_TRY(p->q.alloc((size_t)ctas * vmax * SW));
-  SP_TRY(p->masks.alloc((size_t)ctas * vmax * 3));
-  SP_TRY(p->flv.alloc((size_t)ctas * cap));
-  SP_TRY(p->flm.alloc((size_t)ctas * cap));
-  SP_TRY(p->lo.alloc((size_t)ctas * (maxd + 2)));
-  SP_TRY(p->cnt.alloc(ctas + 1));
-  SP_TRY(p->bc.alloc(g->V));
-  SP_TRY(p->srcs.alloc(std::max(1, nsrc) + 2 * (ngraphs + 1) + ngraphs));
-  SP_TRY(p->err.alloc(1));
   SP_TRY(p->fout.alloc(g->V));
-  int32_t* d_srcs = p->srcs.p;
-  int32_t* d_voff = d_srcs + std::max(1, nsrc);
-  int32_t* d_soff = d_voff + ngraphs + 1;
-  int32_t* d_order = d_soff + ngraphs + 1;
-  if (nsrc) SP_CHECK_CUDA(cudaMemcpyAsync(d_srcs, hs.data(), sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, s));
-  SP_CHECK_CUDA(cudaMemcpyAsync(d_voff, voff.data(), sizeof(int32_t) * (ngraphs + 1), cudaMemcpyHostToDevice, s));
-  SP_CHECK_CUDA(cudaMemcpyAsync(d_soff, soff.data(), sizeof(int32_t) * (ngraphs + 1), cudaMemcpyHostToDevice, s));
-  SP_CHECK_CUDA(cudaMemcpyAsync(d_order, order.data(), sizeof(int32_t) * ngraphs, cudaMemcpyHostToDevice, s));
-  const int zg = num_sms() * 8;
-  bc::k_zero<<<zg, 256, 0, s>>>(p->sigma.p, (size_t)ctas * vmax * SW);
-  bc::k_zero<<<zg, 256, 0, s>>>(p->delta.p, (size_t)ctas * vmax * SW / 2);
-  bc::k_zero<<<zg, 256, 0, s>>>(p->masks.p, (size_t)ctas * vmax * 3);
-  bc::k_zero<<<zg, 256, 0, s>>>(p->bc.p, (size_t)g->V);
-  g_launches += 4;
-  SP_CHECK_CUDA(cudaMemsetAsync(p->cnt.p, 0, sizeof(int) * (ctas + 1), s));
-  SP_CHECK_CUDA(cudaMemsetAsync(p->err.p, 0, sizeof(int), s));
-  bc::GraphsArgs a;
-  a.off = g->off.p;
-  a.adj = g->adj.p;
-  a.voff = d_voff;
-  a.soff = d_soff;
-  a.srcs = d_srcs;
-  a.order = d_order;
-  a.G = ngraphs;
-  a.next = p->cnt.p + ctas;
-  a.sigma = p->sigma.p;
-  a.delta = p->delta.p;
-  a.q = p->q.p;
-  a.masks = p->masks.p;
-  a.flv = p->flv.p;
-  a.flm = p->flm.p;
-  a.lo = p->lo.p;
-  a.cnt = p->cnt.p;
-  a.bc = p->bc.p;
-  a.vmax = vmax;
-  a.cap = cap;
-  a.maxd = maxd;
-  a.err = p->err.p;
-  if (C == 1) {
-    if (NW == 2)
-      bc::k_bc_graphs<2><<<teams, bc::CTA_THREADS, 0, s>>>(a);
-    else
-      bc::k_bc_graphs<1><<<teams, bc::CTA_THREADS, 0, s>>>(a);
-  } else {
-    const int grid = teams * C;
-#define SP_BC_CLUSTERS(CC)                                                          \
-  if (NW == 2)                                                                     \
-    bc::k_bc_clusters<2, CC><<<grid, bc::CTA_THREADS, 0, s>>>(a);                  \
-  else                                                                             \
-    bc::k_bc_clusters<1, CC><<<grid, bc::CTA_THREADS, 0, s>>>(a);
-    if (C == 2) {
-      SP_BC_CLUSTERS(2)
-    } else if (C == 4) {
-      SP_BC_CLUSTERS(4)
-    } else {
-      SP_BC_CLUSTERS(8)
+  // All graphs at once as one graph, the k-th sources of every graph in column k: the whole
+  // GPU shares every level, whatever the graphs' sizes, where a team per graph is bound by
+  // its own latency and the largest graph. 1000 ER graphs of up to 50
+  // thousand vertices, 16 sources each: 34.7 ms against 67; 20 such graphs, 40 sources each:
+  // 1.9 against 58. The union's state must fit;
+  // a set bc.cluster asks for teams.
+  const double state = (double)g->V * (std::min(smax, 64) <= 16 ? 16 : std::min(smax, 64) <= 32 ? 32 : 64) * 16;
+  if (g->bc_cluster <= 0 && nsrc > 0 && state <= bc::UNION_BYTES) {
+    int st = SP_OK;
+    for (int width = std::min(smax, 64);; width = 16) {
+      std::vector<int32_t> order, cols, boff{0};
+      for (int s0 = 0; s0 < smax; s0 += width) {
+        for (int k = 0; k < ngraphs; ++k)
+          for (int j = soff[k] + s0; j < std::min(soff[k + 1], soff[k] + s0 + width); ++j) {
+            order.push_back(hs[j]);
+            cols.push_back(j - soff[k] - s0);
+          }
+        boff.push_back((int)order.size());
+      }
+      SP_TRY(p->srcs.alloc(2 * order.size() + boff.size()));
+      int32_t* d = p->srcs.p;
+      SP_CHECK_CUDA(cudaMemcpyAsync(d, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice, s));
+      SP_CHECK_CUDA(cudaMemcpyAsync(d + order.size(), cols.data(), sizeof(int32_t) * cols.size(),
+                                    cudaMemcpyHostToDevice, s));
+      SP_CHECK_CUDA(cudaMemcpyAsync(d + 2 * order.size(), boff.data(), sizeof(int32_t) * boff.size(),
+                                    cudaMemcpyHostToDevice, s));
+      st = bc_gather(g, d, nsrc, 0, width, maxd, nullptr, nullptr, d + order.size(), d + 2 * order.size(),
+                     (int)boff.size() - 1);
+      if (st != SP_ERR_UNSUPPORTED || width <= 16) break;  // full lists: 16 sources a graph always fit
     }
-#undef SP_BC_CLUSTERS
+    if (st != SP_ERR_OOM) {  // without the memory: teams
+      SP_TRY(st);
+      bc::k_to_float<<<num_sms() * 4, 256, 0, s>>>(p->bc.p, p->fout.p, g->V);
+      SP_CHECK_LAUNCH();
+      return copy_out(BC, p->fout.p, sizeof(float) * g->V, s);
+    }
   }
-  SP_CHECK_LAUNCH();
-  int herr = 0;
-  SP_TRY(copy_out(&herr, p->err.p, sizeof(int), s));
-  if (herr) {
-    set_error("sp_bc_graphs: device error %d (1 level lists full, 2 deeper than %d levels)", herr, maxd);
-    return SP_ERR_UNSUPPORTED;
-  }
-  bc::k_to_float<<<num_sms() * 4, 256, 0, s>>>(p->bc.p, p->fout.p, g->V);
-  SP_CHECK_LAUNCH();
-  return copy_out(BC, p->fout.p, sizeof(float) * g->V, s);
+  const int SW = smax > 32 ? 64 : smax > 16 ? 32 : 16;
+  return bc_graph_teams(g, ngraphs, voff, soff, hs, vmax, smax, SW, BC);
 }
 
 namespace sp {
