@@ -19,15 +19,15 @@
 //    singleton rule (a singleton moves to another singleton only if that label is
 //    smaller) keep neighbours from swapping back and forth;
 //  * per-vertex neighbour-community weights by degree bin: up to 64 edges, one warp
-//    with no table (lanes holding one community found by __match_any_sync and summed
-//    by shuffles); up to slots / 2, one CTA with a hash table of up to `slots` entries
+//    (whole weights at level 0: k_move_whole; otherwise with no table, lanes holding one
+//    community found by __match_any_sync and summed by shuffles); up to slots / 2, one CTA with a hash table of up to `slots` entries
 //    in dynamic shared memory (16384 by default; per level, the learned variant may
 //    take 1024, 2048 or 4096, which fit more CTAs per SM); above that, one CTA with a
 //    table in global scratch; FP64 values, shared-memory atomics in the tables;
 //  * vertices binned by degree class and by sub-sweep parity, so a sub-sweep's
 //    kernels read only the vertices that may move in it;
-//  * tot_c with FP64 atomics aggregated per warp over lanes of one community (exact
-//    for integer weights); Q from the total internal weight (a CTA reduction) and
+//  * tot_c with FP64 atomics aggregated per warp over lanes of one community; whole
+//    weights, whose sums are exact, move only the moved vertices' weight (k_apply_tot); Q from the total internal weight (a CTA reduction) and
 //    the tot_c;
 //  * aggregation: communities renumbered densely, external edges emitted at scan
 //    positions with the key c_u * C + c_v, sorted by this library's stable LSD radix
@@ -48,6 +48,7 @@ namespace sp {
 namespace lv {
 constexpr int THREADS = 256;
 constexpr int WARP_DEG = 64;
+
 constexpr int CTA_SLOTS_MAX = 16384;
 constexpr int EMPTY = -1;
 
@@ -212,6 +213,207 @@ __global__ void __launch_bounds__(THREADS) k_move_warp(MoveArgs a) {
   }
 }
 
+// The same choice for level 0 with whole weights, whose sums are exact in any order.
+//  * The neighbours in v's own community (most of them, once communities have formed) are
+//    counted with a ballot; the others, if at most 32, go to one lane each.
+//  * Lanes of one community find each other through a byte table: every lane writes its
+//    number at its community's hash and reads the number that stayed, whose lane has either
+//    the same community (it leads) or another one (the slot is tried again). Nothing is
+//    cleared. __match_any_sync takes a pass per distinct value here: k_move_warp spends 335
+//    warp instructions on a vertex of 32 edges, with a match per 32 edges.
+//  * Gains are compared by kv / W, computed once per vertex and level, where that decides
+//    beyond its rounding; otherwise as everywhere, with the division.
+// SBM 1M, a sub-sweep: k_move_warp 320 us on average, this 180 (its
+// first sweeps, where every neighbour is its own community, 245; the last 143). Issue (half
+// active) and the chain row, comm, tot of a vertex bound it. One lane per vertex, with its
+// neighbours in shared memory, took 314.
+constexpr int FINDB = 512;  // table bytes per warp
+constexpr int WHOLE_CTAS = 5;  // CTAs an SM; SBM 1M 14.1 ms at 4 and 5, 15.8 at 6 (spills)
+struct WholeScratch {
+  int c[32], w[32], sum[64];
+  uint8_t find[FINDB];
+};
+
+// The best of the lanes' candidates c with gain g (the lanes of on) and v's choice. Gains
+// are compared as integers in the order of their values, high words first.
+__device__ __forceinline__ void best_exact(const MoveArgs& a, int v, int cv, double kv, bool on, int c, double g) {
+  const unsigned FULL = 0xffffffffu;
+  const unsigned long long raw = (unsigned long long)__double_as_longlong(g + 0.0);  // no negative zero
+  const unsigned long long key = raw ^ ((raw >> 63) ? ~0ull : 1ull << 63);
+  const unsigned kh = on ? (unsigned)(key >> 32) : 0u, bh = __reduce_max_sync(FULL, kh);
+  on = on && kh == bh;
+  const unsigned kl = on ? (unsigned)key : 0u, bl = __reduce_max_sync(FULL, kl);
+  on = on && kl == bl;
+  const unsigned id = __reduce_min_sync(FULL, on ? (c == cv ? 0u : (unsigned)c + 1u) : ~0u);
+  if ((threadIdx.x & 31) == 0) {
+    const unsigned long long k = ((unsigned long long)bh << 32) | bl;
+    const double best = __longlong_as_double((long long)(k ^ ((k >> 63) ? 1ull << 63 : ~0ull)));
+    a.newcomm[v] = decide(a, cv, kv, a.tot[cv], a.csize[cv], best, id ? (int)(id - 1u) : cv);
+  }
+}
+
+template <bool UNIT>
+__global__ void __launch_bounds__(THREADS, WHOLE_CTAS) k_move_whole(MoveArgs a, const double* __restrict__ kvW) {
+  __shared__ WholeScratch s_all[THREADS / 32];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  WholeScratch& S = s_all[threadIdx.x >> 5];
+  const unsigned lt = (1u << lane) - 1u;
+  const int gw = (blockIdx.x * THREADS + threadIdx.x) >> 5, nw = (gridDim.x * THREADS) >> 5;
+  // the next vertex's row and community, and the one after it, are loaded ahead
+  int vn = gw < a.nlist ? a.list[gw] : 0, vnn = gw + nw < a.nlist ? a.list[gw + nw] : 0;
+  int bn = a.L.off[vn], en = a.L.off[vn + 1], cn = a.comm[vn];
+  for (int i = gw; i < a.nlist; i += nw) {
+    const int v = vn, b = bn, e = en, cv = cn;
+    const double kv = a.kv[v], r = kvW[v], tot_cv = a.tot[cv];
+    vn = vnn;
+    if (i + nw < a.nlist) {
+      bn = a.L.off[vn];
+      en = a.L.off[vn + 1];
+      cn = a.comm[vn];
+    }
+    if (i + 2 * nw < a.nlist) vnn = a.list[i + 2 * nw];
+    const int j0 = b + lane, j1 = b + 32 + lane;
+    const int u0 = j0 < e ? a.L.adj[j0] : -1, u1 = j1 < e ? a.L.adj[j1] : -1;
+    int w = 1, wb = 1;
+    if (!UNIT) {
+      w = j0 < e ? (int)a.L.w[j0] : 0;
+      wb = j1 < e ? (int)a.L.w[j1] : 0;
+    }
+    int c = u0 >= 0 ? a.comm[u0] : -1, cb = u1 >= 0 ? a.comm[u1] : -1;
+    bool on = c >= 0 && c != cv, onb = cb >= 0 && cb != cv;
+    const unsigned x0 = __ballot_sync(FULL, on), x1 = __ballot_sync(FULL, onb);
+    const int n0 = __popc(x0), nx = n0 + __popc(x1);
+    const int own_n = e - b - nx;
+    if (nx == 0) {  // no other community to go to
+      if (lane == 0) a.newcomm[v] = cv;
+      continue;
+    }
+    const double rest = tot_cv - kv;  // of v's own community
+    int own_w = own_n;
+    if (!UNIT) own_w = __reduce_add_sync(FULL, (c == cv ? w : 0) + (cb == cv ? wb : 0));
+    __syncwarp();
+    if (nx < 32) {
+      if (x1) {
+        if (on) {
+          S.c[__popc(x0 & lt)] = c;
+          if (!UNIT) S.w[__popc(x0 & lt)] = w;
+        }
+        if (onb) {
+          S.c[n0 + __popc(x1 & lt)] = cb;
+          if (!UNIT) S.w[n0 + __popc(x1 & lt)] = wb;
+        }
+        __syncwarp();
+        on = lane < nx;
+        if (on) {
+          c = S.c[lane];
+          if (!UNIT) w = S.w[lane];
+        }
+      }
+      S.sum[lane] = 0;
+      // leaders of equal communities, and their sums
+      uint8_t* slot = S.find + (((unsigned)c * 2654435761u) >> 23);
+      bool todo = on;
+      int lead = lane;
+      do {
+        if (todo) *slot = (uint8_t)lane;
+        __syncwarp();
+        if (todo) lead = *slot;
+        const int lc = __shfl_sync(FULL, c, lead);
+        todo = todo && lc != c;
+      } while (__any_sync(FULL, todo));
+      if (on) atomicAdd(&S.sum[lead], w);
+      __syncwarp();
+      on = on && lead == lane;
+      w = S.sum[lane];
+      double tc = on ? a.tot[c] : 0.0;
+      // v's own community is a candidate too, on a lane that is free
+      const unsigned free1 = __ballot_sync(FULL, !on);
+      if (own_n > 0 && lane == __ffs(free1) - 1) {
+        on = true;
+        c = cv;
+        w = own_w;
+        tc = rest;
+      }
+      // by r: what the best is, if it stands out beyond rounding
+      const double ga = (double)w - tc * r;
+      const int gh = __double2hiint(ga);
+      const unsigned hi = on ? (unsigned)gh ^ ((unsigned)(gh >> 31) | 0x80000000u) : 0u;
+      const unsigned top = __ballot_sync(FULL, hi + 1u >= __reduce_max_sync(FULL, hi) && on);
+      const int l = __ffs(top) - 1;
+      const double bg = __shfl_sync(FULL, ga, l), stay = -(rest * r);
+      const int bc = __shfl_sync(FULL, c, l);
+      // no weight is negative, so no w and no tc * r is above kv: both forms of a gain are
+      // within 4e-15 kv of each other, and gains whose high words differ by two or more are
+      // further apart than that where the larger is above 1e-7 kv
+      if (__popc(top) == 1 && fabs(bg) > 1e-7 * kv && fabs(bg - stay) > 1e-12 * kv) {  // the same for the warp
+        if (lane == 0) {
+          int to = bg > stay ? bc : cv;
+          if (to > cv && a.csize[cv] == 1 && a.csize[to] == 1) to = cv;  // singleton rule
+          a.newcomm[v] = to;
+        }
+        continue;
+      }
+      best_exact(a, v, cv, kv, on, c, (double)w - tc * kv / a.W);
+      continue;
+    }
+    // 32 others and more: a lane may hold two neighbours, the second with number 32 + lane
+    S.sum[lane] = S.sum[32 + lane] = 0;
+    const unsigned h = ((unsigned)c * 2654435761u) >> 23, hb = ((unsigned)cb * 2654435761u) >> 23;
+    bool todo = on, todob = onb;
+    int lead = lane, leadb = 32 + lane;
+    do {
+      if (todo) S.find[h] = (uint8_t)lane;
+      if (todob) S.find[hb] = (uint8_t)(32 + lane);
+      __syncwarp();
+      if (todo) lead = S.find[h];
+      if (todob) leadb = S.find[hb];
+      const int l0 = __shfl_sync(FULL, c, lead & 31), l1 = __shfl_sync(FULL, cb, lead & 31);
+      const int m0 = __shfl_sync(FULL, c, leadb & 31), m1 = __shfl_sync(FULL, cb, leadb & 31);
+      todo = todo && (lead >= 32 ? l1 : l0) != c;
+      todob = todob && (leadb >= 32 ? m1 : m0) != cb;
+    } while (__any_sync(FULL, todo || todob));
+    if (on) atomicAdd(&S.sum[lead], w);
+    if (onb) atomicAdd(&S.sum[leadb], wb);
+    __syncwarp();
+    on = on && lead == lane;
+    onb = onb && leadb == 32 + lane;
+    w = S.sum[lane];
+    wb = S.sum[32 + lane];
+    // v's own community on a lane free for a second one, or, if there is none, for a first
+    // (not all of 64 edges are the others')
+    if (own_n > 0) {
+      const unsigned free2 = __ballot_sync(FULL, !onb), free1 = __ballot_sync(FULL, !on);
+      if (free2) {
+        if (lane == __ffs(free2) - 1) {
+          onb = true;
+          cb = cv;
+          wb = own_w;
+        }
+      } else if (lane == __ffs(free1) - 1) {
+        on = true;
+        c = cv;
+        w = own_w;
+      }
+    }
+    double g1 = 0.0;
+    if (on) g1 = (double)w - (c == cv ? rest : a.tot[c]) * kv / a.W;
+    if (onb) {
+      const double g2 = (double)wb - (cb == cv ? rest : a.tot[cb]) * kv / a.W;
+      if (!on || better(g2, cb, g1, c, cv)) {
+        on = true;
+        g1 = g2;
+        c = cb;
+      }
+    }
+    best_exact(a, v, cv, kv, on, c, g1);
+  }
+}
+
+__global__ void k_ratio(int n, const double* __restrict__ kv, double W, double* __restrict__ kvW) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) kvW[v] = kv[v] / W;
+}
+
 // Plain form (SP_LV_PLAIN): one thread per vertex of the sub-sweep's parity and no
 // tables. Each neighbour community is scored once, at the first neighbour carrying it,
 // and its weight k_{v,c} is found by rescanning the neighbour list: O(deg^2) work per
@@ -339,17 +541,58 @@ __global__ void k_init_comm(int n, int32_t* comm, int32_t* newcomm) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) comm[v] = newcomm[v] = v;
 }
 
-__global__ void k_apply(int n, int parity, int32_t* comm, const int32_t* __restrict__ newcomm, int* moved) {
-  int local = 0;
+__global__ void k_apply(int n, int parity, int32_t* comm, const int32_t* __restrict__ newcomm) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
     if ((int)(hmix((unsigned)v) & 1u) != parity) continue;
-    if (comm[v] != newcomm[v]) {
-      comm[v] = newcomm[v];
-      ++local;
+    if (comm[v] != newcomm[v]) comm[v] = newcomm[v];
+  }
+}
+
+// k_apply for whole weights: the moved vertices' k_v go from the old community's tot to the
+// new one's (exact in FP64, so tot is what k_tot gives), and csize with them. Lanes of a
+// warp that leave or join the same community add up first: in the sweeps that form the
+// large communities one atomic per vertex took up to 137 us, now 38; where no target is
+// shared, the sums are skipped (all 44 calls of SBM 1M: 0.71 ms; always summed 1.06, never 1.09).
+__device__ __forceinline__ void add_group(bool on, int c, double k, double* tot, int32_t* csize, int sign) {
+  const int lane = threadIdx.x & 31;
+  const unsigned grp = __match_any_sync(0xffffffffu, on ? c : -1 - lane);
+  double sum = 0.0;
+  for (unsigned m = grp; m; m &= m - 1) sum += __shfl_sync(grp, k, __ffs(m) - 1);
+  if (on && lane == __ffs(grp) - 1) {
+    atomicAdd(&tot[c], sign * sum);
+    atomicAdd(&csize[c], sign * __popc(grp));
+  }
+}
+
+__global__ void k_apply_tot(int n, int parity, int32_t* comm, const int32_t* __restrict__ newcomm,
+                            const double* __restrict__ kv, double* tot, int32_t* csize) {
+  const int n32 = (n + 31) & ~31;  // every lane of a warp runs the same iterations
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n32; v += gridDim.x * blockDim.x) {
+    int c = 0, d = 0;
+    if (v < n && (int)(hmix((unsigned)v) & 1u) == parity) {
+      c = comm[v];
+      d = newcomm[v];
+    }
+    const bool on = c != d;
+    if (!__any_sync(0xffffffffu, on)) continue;
+    double k = 0.0;
+    if (on) {
+      comm[v] = d;
+      k = kv[v];
+    }
+    // some lanes share a target: add up first
+    const int lead = __ffs(__ballot_sync(0xffffffffu, on)) - 1;
+    const int dl = __shfl_sync(0xffffffffu, d, lead);
+    if (__popc(__ballot_sync(0xffffffffu, on && d == dl)) >= 3) {
+      add_group(on, c, k, tot, csize, -1);
+      add_group(on, d, k, tot, csize, 1);
+    } else if (on) {
+      atomicAdd(&tot[c], -k);
+      atomicAdd(&tot[d], k);
+      atomicAdd(&csize[c], -1);
+      atomicAdd(&csize[d], 1);
     }
   }
-  local = warp_sum(local);
-  if ((threadIdx.x & 31) == 0 && local) atomicAdd(moved, local);
 }
 
 // tot_c = sum of k_v and csize_c = members, per community. Lanes of a warp that hold
@@ -377,14 +620,23 @@ __global__ void k_tot(int n, const int32_t* __restrict__ comm, const double* __r
 // sum_c in_c = sum_v (weight of v's edges inside its community + its self-loop):
 // one partial per CTA, no per-community atomics; the host adds the partials of both
 // kernels in CTA order, so Q is the same on every run. A warp takes 32 vertices at a
-// time and spreads their edges over its lanes (an exclusive scan of the degrees), four
+// time and spreads their edges over its lanes (an exclusive scan of the degrees), U
 // 32-edge steps with their loads in flight together: the row walk of one vertex per
 // warp was a chain of dependent loads per vertex (SBM 1M: 318 us per call).
-__global__ void __launch_bounds__(THREADS) k_internal(Level L, const int32_t* __restrict__ comm, double W,
+// HALF (symmetric graph, unit weights): an edge to a larger vertex counts twice, one to a
+// smaller vertex is not looked up. 113 us before (whole, rows found by a search over the
+// lanes); now 96 at 3 steps and 6 CTAs an SM, 105 at 4 and 6, 110 at 2 and 8, 144 at 6 and 4:
+// latency of adj (read from DRAM each time) and comm bounds it.
+constexpr int INTERNAL_CTAS = 6;
+template <bool HALF>
+__global__ void __launch_bounds__(THREADS, INTERNAL_CTAS) k_internal(Level L, const int32_t* __restrict__ comm, double W,
                                                       double* q) {
-  constexpr int U = 4;
+  constexpr int U = 3;
   __shared__ double s_red[THREADS / 32];
-  const int lane = threadIdx.x & 31;
+  __shared__ int s_row[THREADS / 32][32], s_com[THREADS / 32][32], s_v[HALF ? THREADS / 32 : 1][32];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned le = FULL >> (31 - lane);
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   double acc = 0;
   for (int base = gw * 32; base < L.n; base += nw * 32) {
@@ -399,36 +651,53 @@ __global__ void __launch_bounds__(THREADS) k_internal(Level L, const int32_t* __
     int inc = d;
 #pragma unroll
     for (int k = 1; k < 32; k <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, inc, k);
+      const int t = __shfl_up_sync(FULL, inc, k);
       if (lane >= k) inc += t;
     }
-    const int total = __shfl_sync(0xffffffffu, inc, 31);
+    const int total = __shfl_sync(FULL, inc, 31);
     const int excl = inc - d;
+    // the rows that have edges, in order; in a window of 32 edges their starts are one bit
+    // each, so an edge's row is the number of starts up to it
+    const unsigned nz = __ballot_sync(FULL, d > 0);
+    if (d > 0) {
+      const int k = __popc(nz & (le >> 1));
+      s_row[wid][k] = b - excl;
+      s_com[wid][k] = cv;
+      if (HALF) s_v[wid][k] = v;
+    }
+    __syncwarp();
+    int started = -1;
     for (int t0 = 0; t0 < total; t0 += 32 * U) {
       int u[U], cq[U];
       double wq[U];
 #pragma unroll
       for (int q = 0; q < U; ++q) {
+        const unsigned at = (unsigned)(excl - (t0 + 32 * q));
+        const unsigned m = __reduce_or_sync(FULL, d > 0 && at < 32u ? 1u << at : 0u);
+        const int j = started + __popc(m & le);
+        started += __popc(m);
         const int t = t0 + 32 * q + lane;
-        int j = 0;  // the last lane whose edges start at or before t
-#pragma unroll
-        for (int k = 16; k > 0; k >>= 1)
-          if (__shfl_sync(0xffffffffu, excl, j + k) <= t) j += k;
-        const int jb = __shfl_sync(0xffffffffu, b, j);
-        const int je = __shfl_sync(0xffffffffu, excl, j);
-        cq[q] = __shfl_sync(0xffffffffu, cv, j);
         u[q] = -1;
         wq[q] = 0.0;
+        cq[q] = 0;
         if (t < total) {
-          const int k = jb + (t - je);
+          const int k = s_row[wid][j] + t;
+          cq[q] = s_com[wid][j];
           u[q] = L.adj[k];
-          wq[q] = L.unit ? 1.0 : L.w[k];
+          if (HALF) {
+            const int me = s_v[wid][j];
+            wq[q] = u[q] > me ? 2.0 : 1.0;
+            if (u[q] < me) u[q] = -1;
+          } else {
+            wq[q] = L.unit ? 1.0 : L.w[k];
+          }
         }
       }
 #pragma unroll
       for (int q = 0; q < U; ++q)
         if (u[q] >= 0 && comm[u[q]] == cq[q]) acc += wq[q];
     }
+    __syncwarp();
   }
   acc = block_sum<THREADS>(acc, s_red);
   if (threadIdx.x == 0) q[blockIdx.x] = acc / W;
@@ -520,9 +789,15 @@ __global__ void k_compose(int n0, int32_t* orig, const int32_t* __restrict__ com
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n0; v += gridDim.x * blockDim.x) orig[v] = newid[comm[orig[v]]];
 }
 
-__global__ void k_f2d(const float* __restrict__ a, double* b, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    b[i] = a ? (double)a[i] : 1.0;
+// Weights to FP64 (1.0 without any); *odd = 1 unless all are whole numbers of [0, 2^20].
+__global__ void k_f2d(const float* __restrict__ a, double* b, int64_t n, int* odd) {
+  bool o = false;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float w = a ? a[i] : 1.0f;
+    o |= !(w == rintf(w) && w >= 0.0f && w <= 1048576.0f);
+    b[i] = (double)w;
+  }
+  if (__any_sync(0xffffffffu, o) && (threadIdx.x & 31) == 0) *odd = 1;
 }
 
 // Vertex lists per (degree class, sub-sweep parity): list 2 * b + parity, b = 0 warp,
@@ -531,12 +806,25 @@ __global__ void k_f2d(const float* __restrict__ a, double* b, int64_t n) {
 __global__ void k_bins(int n, const int32_t* __restrict__ off, int32_t* lists, int* counts, int cap, int cta_deg,
                        const int* __restrict__ sel) {
   if (sel) cta_deg = sel[0] / 2;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const int d = off[v + 1] - off[v];
-    const int b = d <= WARP_DEG ? 0 : (d <= cta_deg ? 1 : 2);
-    const int k = 2 * b + (int)(hmix((unsigned)v) & 1u);
-    const int p = atomicAdd(&counts[k], 1);
-    lists[(size_t)k * cap + p] = v;
+  const int lane = threadIdx.x & 31;
+  const int n32 = (n + 31) & ~31;  // every lane of a warp runs the same iterations
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n32; v += gridDim.x * blockDim.x) {
+    int k = -1;
+    if (v < n) {
+      const int d = off[v + 1] - off[v];
+      const int b = d <= WARP_DEG ? 0 : (d <= cta_deg ? 1 : 2);
+      k = 2 * b + (int)(hmix((unsigned)v) & 1u);
+    }
+    // one counter atomic per list and warp (1M vertices 390 us with one per vertex)
+    for (unsigned left = __ballot_sync(0xffffffffu, k >= 0); left;) {
+      const int kk = __shfl_sync(0xffffffffu, k, __ffs(left) - 1);
+      const unsigned m = __ballot_sync(0xffffffffu, k == kk);
+      int p = 0;
+      if (lane == __ffs(m) - 1) p = atomicAdd(&counts[kk], __popc(m));
+      p = __shfl_sync(0xffffffffu, p, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
+      if (k == kk) lists[(size_t)k * cap + p] = v;
+      left &= ~m;
+    }
   }
 }
 
@@ -547,11 +835,11 @@ struct LvPlan {
   dbuf<int32_t> off[2], adj[2];
   dbuf<double> w[2], sl[2];
   dbuf<int32_t> comm, newcomm, csize, used, newid, cnt, pos, orig, lists, rowcnt;
-  dbuf<double> kv, tot, scal, qpart;
+  dbuf<double> kv, tot, scal, qpart, kvW;
   dbuf<unsigned long long> keys, skeys;
   dbuf<double> vals, svals;
   dbuf<int32_t> head, ridx, rstart, scr;
-  dbuf<int> icnt;  // [0, 6) bin sizes, [6] moves applied, [8 ..) the level's variant (lv::SEL)
+  dbuf<int> icnt;  // [0, 6) bin sizes ([0] first: odd weights), [8 ..) the level's variant (lv::SEL)
   dbuf<unsigned long long> vacc;  // the level's degree statistics
   dbuf<float> vmodel;             // the variant model on the device, generation vmodel_gen
   unsigned vmodel_gen = 0;
@@ -573,11 +861,14 @@ int read_int(const int* d, int* h, cudaStream_t s) { return copy_out(h, d, sizeo
 
 }  // namespace
 
-static int lv_modularity(LvPlan* p, const lv::Level& L, double W, cudaStream_t s, double* q) {
+static int lv_modularity(LvPlan* p, const lv::Level& L, double W, bool half, cudaStream_t s, double* q) {
   const int n = L.n;
-  const int g = num_sms() * 8;
+  const int g = num_sms() * lv::INTERNAL_CTAS;
   SP_TRY(p->qpart.alloc(2 * (size_t)g));
-  lv::k_internal<<<g, lv::THREADS, 0, s>>>(L, p->comm.p, W, p->qpart.p);
+  if (half)
+    lv::k_internal<true><<<g, lv::THREADS, 0, s>>>(L, p->comm.p, W, p->qpart.p);
+  else
+    lv::k_internal<false><<<g, lv::THREADS, 0, s>>>(L, p->comm.p, W, p->qpart.p);
   SP_CHECK_LAUNCH();
   lv::k_q<<<g, lv::THREADS, 0, s>>>(n, p->tot.p, W, p->qpart.p + g);
   SP_CHECK_LAUNCH();
@@ -602,7 +893,7 @@ static int lv_recount(LvPlan* p, int n, cudaStream_t s) {
 // = entries of list (b, parity); the global tables of parity 1's big list follow
 // parity 0's in gtab_off.
 static int lv_subsweep(LvPlan* p, lv::MoveArgs a, const int counts[6], int cap, int parity, bool plain,
-                       int slots, cudaStream_t s) {
+                       int slots, bool whole, cudaStream_t s) {
   a.parity = parity;
   if (plain) {
     const int tb = 512;  // the generated code's launch shape (backend_cuda/dsl_cpp_generator.cpp:56-77)
@@ -615,7 +906,16 @@ static int lv_subsweep(LvPlan* p, lv::MoveArgs a, const int counts[6], int cap, 
   if (counts[0 + parity]) {
     a.list = list(0);
     a.nlist = counts[0 + parity];
-    lv::k_move_warp<<<g, lv::THREADS, 0, s>>>(a);
+    if (whole) {
+      // one wave: a warp takes its vertices in turn
+      const int gw = std::min(num_sms() * lv::WHOLE_CTAS, (a.nlist + lv::THREADS / 32 - 1) / (lv::THREADS / 32));
+      if (a.L.unit)
+        lv::k_move_whole<true><<<gw, lv::THREADS, 0, s>>>(a, p->kvW.p);
+      else
+        lv::k_move_whole<false><<<gw, lv::THREADS, 0, s>>>(a, p->kvW.p);
+    } else {
+      lv::k_move_warp<<<g, lv::THREADS, 0, s>>>(a);
+    }
     SP_CHECK_LAUNCH();
   }
   if (counts[2 + parity]) {
@@ -765,7 +1065,9 @@ extern "C" int sp_louvain(sp_graph_h g, const float* weight, double threshold, i
     if (m0) SP_CHECK_CUDA(cudaMemcpyAsync(wtmp.p, weight, sizeof(float) * m0, cudaMemcpyDefault, s));
     dw = wtmp.p;
   }
-  lv::k_f2d<<<gs, 256, 0, s>>>(dw, p->w[0].p, m0);
+  SP_TRY(p->icnt.alloc(32));
+  SP_CHECK_CUDA(cudaMemsetAsync(p->icnt.p, 0, sizeof(int), s));
+  lv::k_f2d<<<gs, 256, 0, s>>>(dw, p->w[0].p, m0, p->icnt.p);
   SP_CHECK_LAUNCH();
   SP_CHECK_CUDA(cudaMemsetAsync(p->sl[0].p, 0, sizeof(double) * n0, s));
   SP_TRY(p->comm.alloc(n0));
@@ -781,7 +1083,6 @@ extern "C" int sp_louvain(sp_graph_h g, const float* weight, double threshold, i
   SP_TRY(p->kv.alloc(n0));
   SP_TRY(p->tot.alloc(n0));
   SP_TRY(p->scal.alloc(2));
-  SP_TRY(p->icnt.alloc(32));
   lv::k_init_comm<<<gs, 256, 0, s>>>(n0, p->orig.p, p->newcomm.p);  // orig[v] = v
   SP_CHECK_LAUNCH();
 
@@ -792,7 +1093,11 @@ extern "C" int sp_louvain(sp_graph_h g, const float* weight, double threshold, i
   lv::k_kv<<<gs, 256, 0, s>>>(L, p->kv.p, p->scal.p + 1);
   SP_CHECK_LAUNCH();
   double W = 0;
+  int odd = 0;
+  SP_CHECK_CUDA(cudaMemcpyAsync(&odd, p->icnt.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   SP_TRY(copy_out(&W, p->scal.p + 1, sizeof(double), s));
+  // whole weights: every sum of them is exact, whatever its order (2^31 of 2^20 at most)
+  const bool whole = !odd;
   if (!(W > 0)) {
     *modularity = 0.0;
     if (levels_out) *levels_out = 0;
@@ -805,6 +1110,14 @@ extern "C" int sp_louvain(sp_graph_h g, const float* weight, double threshold, i
     return SP_OK;
   }
 
+  if (whole && !plain) {
+    SP_TRY(p->kvW.alloc(n0));
+    lv::k_ratio<<<gs, 256, 0, s>>>(n0, p->kv.p, W, p->kvW.p);
+    SP_CHECK_LAUNCH();
+  }
+  // where the symmetry is known, or cheap to learn
+  if (!weight && !plain && g->has_rev) SP_TRY(ensure_symmetry(g));
+  const bool half = !weight && !plain && g->symmetric == 1;
   int cur = 0, levels = 0;
   double qcur = 0;
   const int max_levels = 32, max_sweeps = 100;
@@ -820,7 +1133,7 @@ extern "C" int sp_louvain(sp_graph_h g, const float* weight, double threshold, i
     }
     SP_TRY(lv_recount(p, n, s));
     double qlev0 = 0;
-    SP_TRY(lv_modularity(p, L, W, s, &qlev0));
+    SP_TRY(lv_modularity(p, L, W, half && levels == 0, s, &qlev0));
     if (first) qcur = qlev0;
     first = false;
     // kernel variant of this level, chosen on the device (forced, learned, or the
@@ -902,15 +1215,19 @@ extern "C" int sp_louvain(sp_graph_h g, const float* weight, double threshold, i
     double qold = qlev0, qnew = qlev0;
     for (int sweep = 0; sweep < max_sweeps; ++sweep) {
       for (int parity = 0; parity < 2; ++parity) {
-        SP_TRY(lv_subsweep(p, a, counts, n0, parity, plain, slots, s));
-        SP_CHECK_CUDA(cudaMemsetAsync(p->icnt.p + 6, 0, sizeof(int), s));
-        lv::k_apply<<<gs, 256, 0, s>>>(n, parity, p->comm.p, p->newcomm.p, p->icnt.p + 6);
-        SP_CHECK_LAUNCH();
-        SP_TRY(lv_recount(p, n, s));
+        SP_TRY(lv_subsweep(p, a, counts, n0, parity, plain, slots, whole && levels == 0, s));
+        if (whole && !plain) {
+          lv::k_apply_tot<<<gs, 256, 0, s>>>(n, parity, p->comm.p, p->newcomm.p, p->kv.p, p->tot.p, p->csize.p);
+          SP_CHECK_LAUNCH();
+        } else {
+          lv::k_apply<<<gs, 256, 0, s>>>(n, parity, p->comm.p, p->newcomm.p);
+          SP_CHECK_LAUNCH();
+          SP_TRY(lv_recount(p, n, s));
+        }
       }
       qold = qnew;
       ++total_sweeps;
-      SP_TRY(lv_modularity(p, L, W, s, &qnew));
+      SP_TRY(lv_modularity(p, L, W, half && levels == 0, s, &qnew));
       if (!(qnew - qold > threshold)) break;
     }
     if (ev0) {
