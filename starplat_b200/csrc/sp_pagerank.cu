@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "sp_internal.cuh"
+#include "sp_sync.cuh"
 
 namespace sp {
 
@@ -102,6 +103,8 @@ struct PrPlan {
   dspan<double> diff_part;
   dspan<float> prb[2], con[2];
   dspan<pr::State> state;
+  static_assert(sizeof(GridBar) <= sizeof(pr::State), "the barrier fits in the second State");
+  GridBar* bar() const { return (GridBar*)(state.p + 1); }  // k_run
   int hot = -1;           // hot id count the plan was built for
   int order = 0;          // vertex order (k_deg_keys)
   int nparts = 1, part_idx = 0;  // split plan: part part_idx of nparts (lay())
@@ -172,7 +175,7 @@ __device__ __forceinline__ double finalize_row(const IterArgs& a, int r, double 
                                                float* __restrict__ con_new) {
   const float s = (float)sum;
   const float np = __fadd_rn(a.base, __fmul_rn(a.delta, s));
-  const float po = pr_old[r];
+  const float po = __ldcg(pr_old + r);
   pr_new[r] = np;
   const int od = a.od[r];
   con_new[r] = od > 0 ? __fdiv_rn(np, (float)od) : 0.0f;
@@ -236,6 +239,22 @@ struct GatherGlobal {
       return v;
     }
     return __ldg(con + u);
+  }
+};
+// The same within one launch of all iterations (k_run): contrib changes between the
+// barriers, so its loads are not read-only ones.
+template <int SH, int GH>
+struct GatherLive {
+  static constexpr int kSrcHint = SH;
+  const float* con;
+  int hot;
+  __device__ __forceinline__ float operator()(int u) const {
+    float v;
+    if (GH == 1 && u >= hot)
+      asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(con + u));
+    else
+      asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(con + u));
+    return v;
   }
 };
 // Sum of con[radj[i]] for i in [b, e) by a group of W lanes (sl = lane within the
@@ -328,13 +347,13 @@ __device__ __forceinline__ double warp_task(const IterArgs& a, int start, int co
   return finalize_row(a, r, sum, pr_old, pr_new, con_new);
 }
 
-// One phase of one iteration by persistent CTAs of NT threads: long-row chunks
-// first (a CTA each, CHUNK / NT loads per thread), then the warp tasks, heaviest
-// bins first; then the diff partials (the last CTA of the cold phase sums them).
+// The rows of one phase of one iteration by persistent CTAs of NT threads: long-row
+// chunks first (a CTA each, CHUNK / NT loads per thread), then the warp tasks, heaviest
+// bins first. Returns this thread's part of the diff.
 template <int PH, int NT, int VEC, class G>
-__device__ __forceinline__ void phase_body(const IterArgs& a, const G& gather, const float* __restrict__ pr_old,
-                                           float* __restrict__ pr_new, float* __restrict__ con_new, double* s_red,
-                                           int& s_last) {
+__device__ __forceinline__ double phase_work(const IterArgs& a, const G& gather,
+                                             const float* __restrict__ pr_old, float* __restrict__ pr_new,
+                                             float* __restrict__ con_new, double* s_red, int& s_last) {
   constexpr int CI = CHUNK / NT;
   static_assert(CI * NT == CHUNK, "chunk must be a multiple of the CTA size");
   const int tid = threadIdx.x;
@@ -418,7 +437,17 @@ __device__ __forceinline__ void phase_body(const IterArgs& a, const G& gather, c
     }
   }
 
-  const double bd = block_sum<NT>(my_diff, s_red);
+  return my_diff;
+}
+
+// One phase of one iteration: its rows, then the diff partials (the last CTA of the cold
+// phase sums them).
+template <int PH, int NT, int VEC, class G>
+__device__ __forceinline__ void phase_body(const IterArgs& a, const G& gather, const float* __restrict__ pr_old,
+                                           float* __restrict__ pr_new, float* __restrict__ con_new, double* s_red,
+                                           int& s_last) {
+  const int tid = threadIdx.x;
+  const double bd = block_sum<NT>(phase_work<PH, NT, VEC>(a, gather, pr_old, pr_new, con_new, s_red, s_last), s_red);
   if (PH == 0) {
     if (tid == 0) a.diff_part[blockIdx.x] = bd;
     return;
@@ -461,6 +490,69 @@ __global__ void __launch_bounds__(THREADS, 8) k_phase(IterArgs a, const float* _
   __shared__ int s_last;
   if (a.st->done) return;
   phase_body<PH, THREADS, VEC>(a, GatherGlobal<SH, GH>{con_old, a.l1_hot}, pr_old, pr_new, con_new, s_red, s_last);
+}
+
+// All iterations in one cooperative launch, then the ranks in the caller's vertex order:
+// one grid barrier per iteration, after which every CTA adds up the CTAs' diff partials in
+// the same order and takes the same decision. A graph of max_iter launches ran to its end
+// however early the stop test held, 2.5 us and more for each of 100 launches: ER 1,000 of
+// degree 16 219 us a call, now 69; ER 100,003 283, now 159; R-MAT 16 795, now 722. On
+// large graphs the iteration's own time decides, and there k_phase is faster (its loads of
+// contrib are read-only ones, its occupancy is twice this): R-MAT 18 1.13 ms against 1.24,
+// R-MAT 22 11.6 against 12.8 (8 CTAs an SM) to 18.8 (3). So it runs up to RUN_MAX_E in-edges
+// (ER 300,000: 4.8 M, 422 -> 358 us), or RUN_MAX_LONG_E where rows are split in chunks.
+constexpr int RUN_CTAS = 4;
+constexpr int64_t RUN_MAX_E = 6000000, RUN_MAX_LONG_E = 1500000;
+struct RunBufs {
+  float* pr[2];
+  float* con[2];
+  const int32_t* __restrict__ zrows;  // rows without in-edges, written in iterations 0 and 1
+  int nz;
+  GridBar* bar;
+  const int32_t* __restrict__ new_id;
+  float* out;
+  int V;
+};
+
+template <int SH, int GH, int VEC>
+__global__ void __launch_bounds__(THREADS, RUN_CTAS) k_run(IterArgs a, RunBufs b) {
+  __shared__ double s_red[THREADS / 32];
+  __shared__ int s_last;
+  const int t = blockIdx.x * THREADS + threadIdx.x, nt = gridDim.x * THREADS;
+  int k = 0;
+  while (true) {
+    const float* pr_old = b.pr[k & 1];
+    float* pr_new = b.pr[(k & 1) ^ 1];
+    float* con_new = b.con[(k & 1) ^ 1];
+    double d = 0;
+    if (k < 2)
+      for (int i = t; i < b.nz; i += nt) {
+        const int r = b.zrows[i];
+        d += fabs((double)a.base - (double)__ldcg(pr_old + r));
+        pr_new[r] = a.base;
+        const int od = a.od[r];
+        con_new[r] = od > 0 ? __fdiv_rn(a.base, (float)od) : 0.0f;
+      }
+    d += phase_work<1, THREADS, VEC>(a, GatherLive<SH, GH>{b.con[k & 1], a.l1_hot}, pr_old, pr_new, con_new, s_red,
+                                     s_last);
+    d = block_sum<THREADS>(d, s_red);
+    double* part = a.diff_part + (size_t)(k & 1) * gridDim.x;  // the other half may still be read
+    if (threadIdx.x == 0) part[blockIdx.x] = d;
+    if (!grid_barrier(b.bar)) return;
+    double p = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += THREADS) p += __ldcg(part + i);
+    const double all = block_sum<THREADS>(p, s_red);
+    ++k;
+    if (all > a.beta && k < a.max_iter) continue;
+    if (t == 0) {
+      a.st->iter = k;
+      a.st->diff = all;
+      a.st->done = 1;
+    }
+    break;
+  }
+  const float* ranks = b.pr[k & 1];
+  for (int v = t; v < b.V; v += nt) b.out[v] = __ldcg(ranks + b.new_id[v]);
 }
 
 // Rows without in-edges, iterations 0 and 1 only: pr' = (1-delta)/V. Their diff
@@ -736,6 +828,8 @@ __global__ void k_init(int V, const int32_t* __restrict__ odeg, float* __restric
     st->ticket = 0;
     st->diff = 0;
     st->extra = 0;
+    ((GridBar*)(st + 1))->arrived = 0;
+    ((GridBar*)(st + 1))->error = 0;
   }
 }
 
@@ -757,6 +851,8 @@ __global__ void k_init_from(int V, const int32_t* __restrict__ new_id, const int
     st->ticket = 0;
     st->diff = 0;
     st->extra = 0;
+    ((GridBar*)(st + 1))->arrived = 0;
+    ((GridBar*)(st + 1))->error = 0;
   }
 }
 
@@ -833,7 +929,7 @@ static int relabel(sp_graph* g, PrPlan* p) {
   A.want(p->hot_end, Vp);
   A.want(p->part, Vp);
   A.want(p->diff_part, 2 * (size_t)num_sms() * 32);
-  A.want(p->state, 1);
+  A.want(p->state, 2);  // the second holds k_run's barrier
   for (int i = 0; i < 2; ++i) {
     A.want(p->prb[i], Vp);
     A.want(p->con[i], Vp);
@@ -1234,8 +1330,17 @@ static int pr_tuned(sp_graph* g, float beta, float delta, int32_t maxIter, float
       {{pr::k_phase<1, 1, 0, 0>, pr::k_phase<1, 1, 0, 1>}, {pr::k_phase<1, 1, 1, 0>, pr::k_phase<1, 1, 1, 1>}},
       {{pr::k_phase<1, 2, 0, 0>, pr::k_phase<1, 2, 0, 1>}, {pr::k_phase<1, 2, 1, 0>, pr::k_phase<1, 2, 1, 1>}}};
   const PhaseFn ph1 = table[sh][gh][vec];
+  using RunFn = void (*)(pr::IterArgs, pr::RunBufs);
+  static const RunFn runs[3][2][2] = {
+      {{pr::k_run<0, 0, 0>, pr::k_run<0, 0, 1>}, {pr::k_run<0, 1, 0>, pr::k_run<0, 1, 1>}},
+      {{pr::k_run<1, 0, 0>, pr::k_run<1, 0, 1>}, {pr::k_run<1, 1, 0>, pr::k_run<1, 1, 1>}},
+      {{pr::k_run<2, 0, 0>, pr::k_run<2, 0, 1>}, {pr::k_run<2, 1, 0>, pr::k_run<2, 1, 1>}}};
+  const RunFn run = runs[sh][gh][vec];
   const int exec_key = sh | (vec << 2) | (l1_hot << 3);
-  SP_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ph1, pr::THREADS, 0));
+  // one launch for all iterations where the launches would cost more than it does
+  const bool whole = !a.two_phase && g->E <= (p->n_chunks[1] ? pr::RUN_MAX_LONG_E : pr::RUN_MAX_E);
+  const void* fn = whole ? (const void*)run : (const void*)ph1;
+  SP_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, pr::THREADS, 0));
   const int grid = std::max(1, std::min(num_sms() * 32, num_sms() * std::max(1, per_sm)));
   if (init) {
     SP_CHECK_CUDA(cudaMemcpyAsync(p->outbuf.p, init, sizeof(float) * V, cudaMemcpyDefault, s));
@@ -1245,6 +1350,36 @@ static int pr_tuned(sp_graph* g, float beta, float delta, int32_t maxIter, float
     pr::k_init<<<num_sms() * 4, 256, 0, s>>>(V, p->od.p, p->prb[0].p, p->con[0].p, p->state.p);
   }
   SP_CHECK_LAUNCH();
+  if (whole) {
+    pr::RunBufs b;
+    for (int k = 0; k < 2; ++k) {
+      b.pr[k] = p->prb[k].p;
+      b.con[k] = p->con[k].p;
+    }
+    b.zrows = p->zrows;
+    b.nz = p->n_zero;
+    b.bar = p->bar();
+    b.new_id = p->new_id.p;
+    b.out = p->outbuf.p;
+    b.V = V;
+    // a small graph's barriers wait for as few CTAs as have work
+    const long long want =
+        std::max<long long>((long long)p->n_chunks[1] + (p->task_base[1][4] + 7) / 8, (V + 2047) / 2048);
+    const int ctas = (int)std::max<long long>(1, std::min<long long>(grid, want));
+    void* params[] = {&a, &b};
+    SP_CHECK_CUDA(cudaLaunchCooperativeKernel((const void*)run, ctas, pr::THREADS, params, 0, s));
+    g_launches++;
+    if (out) SP_CHECK_CUDA(cudaMemcpyAsync(out, p->outbuf.p, sizeof(float) * V, cudaMemcpyDefault, s));
+    pr::State st[2];
+    SP_TRY(copy_out(st, p->state.p, sizeof(st), s));
+    if (((const GridBar*)(st + 1))->error) {
+      set_error("sp_pagerank: grid barrier timed out");
+      return SP_ERR_TIMEOUT;
+    }
+    if (iters) *iters = st[0].iter;
+    if (fdiff) *fdiff = st[0].diff;
+    return SP_OK;
+  }
   // the iterations: every kernel returns at once after the stop test has ended the run
   auto enqueue = [&](cudaStream_t cs) {
     for (int k = 0; k < n_iter; ++k) {
