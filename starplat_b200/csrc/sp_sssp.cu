@@ -12,14 +12,13 @@
 //     current bucket threshold; far pile F holds the rest;
 //   * relax rounds: every frontier vertex pushes along its out-edges with
 //     atomicMin. A warp holds up to 32 frontier vertices, one per lane, and their
-//     edges are flattened over its lanes (an exclusive scan of the degrees), 32
-//     edges per step, so a 4-neighbour grid vertex costs one step, not four; a
-//     small frontier is spread over all warps. SU steps go together: their dist
-//     loads, atomicMins and mark updates are all issued before any is waited
-//     for, and their queue appends share one counter atomic. Vertices above hub_deg out-edges
-//     (R-MAT hubs) are queued in a hub list whose chunks all warps share in the
-//     next round; queue appends are warp-aggregated and de-duplicated with
-//     per-round / per-epoch mark bitmaps;
+//     edges are flattened over its lanes, 32 edges per window, so a 4-neighbour grid
+//     vertex costs one window, not four; a small frontier is spread over all warps. SU
+//     windows go together: their dist loads and atomicMins are all issued before any is
+//     waited for. Improved vertices gather in the warp's ring in shared memory and are
+//     marked (per-round / per-epoch bitmaps keep a queue free of repeats) and queued 32 at
+//     a time. Vertices above hub_deg out-edges (R-MAT hubs) are queued in a hub list whose
+//     pieces all warps share in the next round;
 //   * warp-local cascades (rounds whose frontier is at most 32 vertices per warp):
 //     a vertex a warp improves below the bucket threshold goes to the warp's ring
 //     in shared memory instead of the next round's queue, and the warp relaxes its
@@ -49,14 +48,17 @@ namespace ss {
 constexpr int THREADS = 256;
 // Queued vertices above HUB_DEG out-edges are relaxed in HUB_CHUNK-edge pieces that
 // every warp shares, so no warp walks a long row alone while the others wait at the
-// round's barrier. R-MAT 23 (learned schedule): 12.6 ms at (2048, 256), 11.5 at
-// (512, 128), 11.2 at (128, 64), 12.0 at (32, 32).
+// round's barrier. A warp takes up to HUB_RUN consecutive pieces as the rows of one batch
+// (a piece alone cost a search of the hub list and three dependent loads for 64 edges).
+// R-MAT 23 / R-MAT 20 at 1 piece a run 5.85 / 0.95 ms, 4: 4.18 / 0.88, 8: 4.02 / 0.90,
+// 32: 4.05 / 1.04 (distances read too long before they are used: more edges relaxed again).
 constexpr int HUB_DEG = 128;
 constexpr int HUB_CHUNK = 64;
+constexpr int HUB_RUN = 8;
 constexpr int HUB_DEG_MAX = 1 << 25;  // 32 entries of at most this degree sum below 2^31
-constexpr int RING = 256;             // entries of a warp's cascade ring (power of two)
+constexpr int RING = 256;             // entries of a warp's rings (a power of two above 31 + 32 * SU)
 constexpr int LOCAL_STEPS = 64;       // default cascade budget: 32-edge warp steps per round
-constexpr int SU = 4;                 // 32-edge steps whose loads and atomics are in flight together
+constexpr int SU = 4;                 // 32-edge windows whose loads and atomics are in flight together
 // Sources per cooperative launch of the batched form. 16 weighted closeness sources of
 // undirected R-MAT 20: 34.1 ms with 1 per launch, 34.5 with 4 or 8, 36.0 with 16.
 constexpr int BATCH = 4;
@@ -137,11 +139,17 @@ struct Out {
   int* fmin;
 };
 
-// A warp's cascade ring in shared memory; head and cnt are warp-uniform.
+// A warp's staging rings in shared memory: improved vertices below the bucket threshold
+// (with their CSR rows in a cascade) and vertices for the far pile. head, cnt, fhead and
+// fcnt are warp-uniform; fmin is the smallest distance this lane sent to the far pile.
+struct RingMem {
+  int32_t v[RING], b[RING], d[RING], far[RING];
+};
 struct Ring {
-  int32_t* s;
-  int head;
-  int cnt;
+  RingMem* s;
+  int head, cnt;
+  int fhead, fcnt;
+  int fmin;
 };
 
 // Adjacency and weights are streamed: each is read once per expansion of its vertex,
@@ -210,257 +218,291 @@ __device__ __forceinline__ void queue_push(const Args& a, bool want, int u, int3
   warp_push(a, want && !hub, u, QN, qnext);
 }
 
-// Below-threshold improvements of this step (want lanes). LOCAL: into the warp's
-// ring while it has room, the rest marked into the next round's queue. Otherwise
-// the caller's relax already marked them: straight into the queue.
-template <bool LOCAL>
-__device__ __forceinline__ void push_near(const Args& a, bool want, int u, int round, const Out& o, Ring& r) {
-  if (LOCAL) {
-    const unsigned m = __ballot_sync(FULL, want);
-    if (!m) return;
-    const int lane = threadIdx.x & 31;
-    const int room = RING - r.cnt;
-    const int rank = __popc(m & ((1u << lane) - 1u));
-    const bool mine = want && rank < room;
-    if (mine) r.s[(r.head + r.cnt + rank) & (RING - 1)] = u;
-    r.cnt += min(__popc(m), room);
-    want = want && !mine && mark(qbits(a, round + 1), u);
+// The improvements of N windows into the warp's ring (b, d: their rows, LOCAL only), as far
+// as it has room; LOCAL marks and queues the rest, and the vertices above hub_deg (the
+// caller keeps room for all of them otherwise).
+template <bool LOCAL, int N>
+__device__ __forceinline__ void ring_push(const Args& a, const bool (&near)[N], const int (&u)[N], const int (&b)[N],
+                                          const int (&d)[N], int round, const Out& o, Ring& r) {
+  const int lane = threadIdx.x & 31;
+  unsigned m[N];
+  int n = 0;
+  bool hub = false;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    m[q] = __ballot_sync(FULL, near[q]);
+    n += __popc(m[q]);
+    if (LOCAL) hub |= near[q] && d[q] > a.hub_deg;
   }
-  queue_push(a, want, u, o.QN, o.qnext, o.HV, o.HB, o.hnext);
+  if (n == 0) return;
+  const unsigned lt = (1u << lane) - 1u;
+  if (!LOCAL || (r.cnt + n <= RING && !__any_sync(FULL, hub))) {
+    int at = r.head + r.cnt;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      if (near[q]) {
+        const int i = (at + __popc(m[q] & lt)) & (RING - 1);
+        r.s->v[i] = u[q];
+        if (LOCAL) {
+          r.s->b[i] = b[q];
+          r.s->d[i] = d[q];
+        }
+      }
+      at += __popc(m[q]);
+    }
+    r.cnt += n;
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    const bool fits = near[q] && d[q] <= a.hub_deg;
+    m[q] = __ballot_sync(FULL, fits);
+    const int rank = __popc(m[q] & lt), room = RING - r.cnt;
+    const bool mine = fits && rank < room;
+    if (mine) {
+      const int i = (r.head + r.cnt + rank) & (RING - 1);
+      r.s->v[i] = u[q];
+      r.s->b[i] = b[q];
+      r.s->d[i] = d[q];
+    }
+    r.cnt += min(__popc(m[q]), room);
+    const bool rest = near[q] && !mine && mark(qbits(a, round + 1), u[q]);
+    queue_push(a, rest, u[q], o.QN, o.qnext, o.HV, o.HB, o.hnext);
+  }
 }
 
-// Relax N edges per lane (nd = dist + weight for target u; nd >= INT_MAX: no edge):
-// every dist load is issued, then every atomicMin, then every mark update, before
-// any result is waited for. res: 1 = improved below the bucket threshold (with
-// STAMP, only the first such improvement of u this round), 2 = improved above it
-// and first in the far pile this epoch, 0 = nothing to queue. When two edges of a
-// group hit the same vertex, the atomics decide; the loads only filter. The dist
-// loads are skipped (every candidate goes to atomicMin) when a.filter is 0, and by
-// default in cascades (!STAMP), where they would add a round trip to each hop: grid
-// 4096^2 33.5 -> 30.6 ms; R-MAT 23 (no cascades) keeps them, where skipping them
-// everywhere measured 6.6 against 6.4 ms. Carrying each ring entry's CSR row, loaded
-// beside the atomicMin, to save the offset load of the next hop measured slower
-// (33.6 ms on the grid).
-template <bool STAMP, int N>
-__device__ __forceinline__ void relax_group(const Args& a, const int (&u)[N], const long long (&nd)[N],
-                                            long long thr, int round, int epoch, int* fmin_slot, int (&res)[N]) {
-  const bool filt = a.filter < 0 ? STAMP : a.filter != 0;
-  int cur[N], old[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-    cur[q] = nd[q] < (long long)INT_MAX ? (filt ? __ldcg(a.dist + u[q]) : INT_MAX) : INT_MIN;
+// The ring's oldest entries (32 at most) to the next round's queue: those that no warp
+// has marked for it yet.
+__device__ __forceinline__ void ring_flush(const Args& a, int round, const Out& o, Ring& r) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  const int take = min(r.cnt, 32);
+  int u = 0;
+  bool want = false;
+  if (lane < take) {
+    u = r.s->v[(r.head + lane) & (RING - 1)];
+    want = mark(qbits(a, round + 1), u);
+  }
+  queue_push(a, want, u, o.QN, o.qnext, o.HV, o.HB, o.hnext);
+  __syncwarp();
+  r.head = (r.head + take) & (RING - 1);
+  r.cnt -= take;
+}
+
+// The same for the far pile.
+__device__ __forceinline__ void far_flush(const Args& a, int epoch, const Out& o, Ring& r) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  const int take = min(r.fcnt, 32);
+  int u = 0;
+  bool want = false;
+  if (lane < take) {
+    u = r.s->far[(r.fhead + lane) & (RING - 1)];
+    want = mark(fbits(a, epoch), u);
+  }
+  warp_push(a, want, u, o.F, o.fcnt);
+  __syncwarp();
+  r.fhead = (r.fhead + take) & (RING - 1);
+  r.fcnt -= take;
+}
+
+// Relaxes N entries per lane: targets u at candidate distances nd (INT_MAX: none). Every
+// load of a kind is issued before any result is waited for. An improvement below the
+// bucket threshold goes to the ring, above it to the far ring, which empties 32 at a time:
+// marking and appending in the step itself cost two more round trips in nearly every step
+// of a cascade. LOCAL loads the targets' rows beside the atomicMins, so that a hop waits
+// for two memory round trips (adjacency, atomicMin) where it waited for three.
+// The dist loads are a filter only (the atomics decide). They are skipped (every
+// candidate goes to atomicMin) when a.filter is 0, and by default in cascades (LOCAL),
+// where they would add a round trip to each hop: grid 4096^2 33.5 -> 30.6 ms; R-MAT 23 (no
+// cascades) keeps them, where skipping them everywhere measured 6.6 against 6.4 ms.
+template <bool LOCAL, int N>
+__device__ __forceinline__ void relax_targets(const Args& a, const int (&u)[N], const int (&nd)[N], int thr,
+                                              int round, int epoch, const Out& o, Ring& r) {
+  const int lane = threadIdx.x & 31;
+  const bool filt = a.filter < 0 ? !LOCAL : a.filter != 0;
+  int old[N], b[N], d[N];
 #pragma unroll
   for (int q = 0; q < N; ++q) {
-    old[q] = INT_MIN;
-    if ((int)nd[q] < cur[q]) old[q] = atomicMin(a.dist + u[q], (int)nd[q]);
+    old[q] = INT_MAX;
+    if (filt && nd[q] != INT_MAX) old[q] = __ldcg(a.dist + u[q]);
   }
 #pragma unroll
   for (int q = 0; q < N; ++q) {
-    res[q] = 0;
-    const int ndi = (int)nd[q];
-    if (ndi < old[q]) {
-      if (nd[q] < thr) {
-        res[q] = (!STAMP || mark(qbits(a, round + 1), u[q])) ? 1 : 0;
-      } else {
-        atomicMin(fmin_slot, ndi);
-        res[q] = mark(fbits(a, epoch), u[q]) ? 2 : 0;
+    const bool go = nd[q] < old[q];
+    old[q] = INT_MIN;
+    b[q] = d[q] = 0;
+    if (go) {
+      old[q] = atomicMin(a.dist + u[q], nd[q]);
+      if (LOCAL) {
+        b[q] = a.off[u[q]];
+        d[q] = a.off[u[q] + 1];
       }
     }
   }
-}
-
-// Appends the flagged values of N steps to buf with one counter atomic per warp.
-template <int N>
-__device__ __forceinline__ void warp_push_many(const Args& a, const bool (&want)[N], const int (&val)[N], int32_t* buf,
-                                               int* counter) {
-  unsigned m[N];
-  int n = 0;
+  bool near[N], far = false;
 #pragma unroll
   for (int q = 0; q < N; ++q) {
-    m[q] = __ballot_sync(FULL, want[q]);
-    n += __popc(m[q]);
+    near[q] = nd[q] < old[q] && nd[q] < thr;
+    far |= nd[q] < old[q] && nd[q] >= thr;
+    d[q] -= b[q];
   }
-  if (n == 0) return;
-  const int lane = threadIdx.x & 31;
-  int base = 0;
-  if (lane == 0) base = atomicAdd(counter, n);
-  base = __shfl_sync(FULL, base, 0);
-  const unsigned lt = (1u << lane) - 1u;
+  ring_push<LOCAL, N>(a, near, u, b, d, round, o, r);
+  if (__any_sync(FULL, far)) {
 #pragma unroll
-  for (int q = 0; q < N; ++q) {
-    if (want[q]) put(a, buf, base + __popc(m[q] & lt), val[q]);
-    base += __popc(m[q]);
-  }
-}
-
-// Next round's queue for N steps: vertices above hub_deg out-edges go to the hub list
-// (their degree loads all issued first), the rest with one counter atomic.
-template <int N>
-__device__ __forceinline__ void queue_push_many(const Args& a, const bool (&want)[N], const int (&u)[N],
-                                                const Out& o) {
-  int nch[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    nch[q] = 0;
-    if (want[q]) {
-      const int d = a.off[u[q] + 1] - a.off[u[q]];
-      if (d > a.hub_deg) nch[q] = (d + a.hub_chunk - 1) / a.hub_chunk;
+    for (int q = 0; q < N; ++q) {
+      const bool f = nd[q] < old[q] && nd[q] >= thr;
+      const unsigned m = __ballot_sync(FULL, f);
+      if (f) {
+        r.fmin = min(r.fmin, nd[q]);
+        r.s->far[(r.fhead + r.fcnt + __popc(m & ((1u << lane) - 1u))) & (RING - 1)] = u[q];
+      }
+      r.fcnt += __popc(m);
     }
+    while (r.fcnt >= 32) far_flush(a, epoch, o, r);  // 31 at most stay: room for 32 * SU more
   }
-  bool nr[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    if (nch[q]) {
-      const unsigned long long old = atomicAdd(o.hnext, (1ull << 32) | (unsigned long long)nch[q]);
-      const int idx = (int)(old >> 32);
-      put(a, o.HV, idx, u[q]);
-      put(a, o.HB, idx, (int)(old & 0xffffffffull));
-    }
-    nr[q] = want[q] && nch[q] == 0;
-  }
-  warp_push_many<N>(a, nr, u, o.QN, o.qnext);
 }
 
-// Pushes of one group: below-threshold improvements to the ring (LOCAL) or the next
-// round's queue, far ones to the far pile.
+// A warp's rows: lane i < n holds the row of d entries from b at distance dv. Lane i's
+// entries take positions [excl, excl + d) of the flattened rows.
+struct Rows {
+  int shift;  // b - excl
+  int excl;
+  int dv;
+  int n;
+  int total;
+};
+
+// Relaxes the N * 32 positions from t0. before: the rows that start below t0. A
+// position's row is the last that starts at or before it; the starts within a window of
+// 32 positions are one bit each of a warp-wide OR, so a lane's row is a count of bits (a
+// search over the lanes' offsets took five dependent shuffles).
 template <bool LOCAL, int N>
-__device__ __forceinline__ void push_group(const Args& a, const int (&res)[N], const int (&u)[N], int round,
-                                           const Out& o, Ring& r) {
-  bool nr[N], fr[N];
+__device__ __forceinline__ void relax_step(const Args& a, const Rows& w, int t0, int& before, int thr, int round,
+                                           int epoch, const Out& o, Ring& r) {
+  const int lane = threadIdx.x & 31;
+  int u[N], nd[N], j[N];
 #pragma unroll
   for (int q = 0; q < N; ++q) {
-    nr[q] = res[q] == 1;
-    fr[q] = res[q] == 2;
-  }
-  if (LOCAL) {
-#pragma unroll
-    for (int q = 0; q < N; ++q) push_near<true>(a, nr[q], u[q], round, o, r);
-  } else {
-    queue_push_many<N>(a, nr, u, o);
-  }
-  warp_push_many<N>(a, fr, u, o.F, o.fcnt);
-}
-
-// Relax the out-edges of the warp's batch: lane i holds frontier vertex v (or -1).
-// Lane i's edges take positions [excl_i, excl_i + d_i) of the flattened batch; in a
-// step, lane t relaxes position t0 + t, owned by the last lane j with excl_j <= t0 + t
-// (a lane of degree 0 is never that last lane). LOCAL also sends vertices above
-// hub_deg (which only the ring can hold) to the next round's hub list. `work` counts
-// the edges relaxed.
-template <bool LOCAL>
-__device__ __forceinline__ void relax_batch(const Args& a, int v, long long thr, int round, int epoch, const Out& o,
-                                            Ring& r, int& work) {
-  const int lane = threadIdx.x & 31;
-  int b = 0, d = 0;
-  long long dv = 0;
-  bool hub = false;
-  if (v >= 0) {
-    // dist[v] is loaded with the offsets, not after the hub test; it is first needed
-    // after the adjacency loads below are issued
-    b = a.off[v];
-    const int e = a.off[v + 1];
-    dv = __ldcg(a.dist + v);
-    d = e - b;
-    if (LOCAL && d > a.hub_deg) {
-      hub = true;
-      d = 0;
+    const int t = t0 + 32 * q + lane;
+    const unsigned p = (unsigned)(w.excl - (t - lane));
+    const unsigned m = __reduce_or_sync(FULL, lane < w.n && p < 32u ? 1u << p : 0u);
+    j[q] = before + __popc(m << (31 - lane)) - 1;
+    before += __popc(m);
+    const int k = __shfl_sync(FULL, w.shift, j[q]) + t;
+    u[q] = nd[q] = 0;
+    if (t < w.total) {
+      u[q] = ld_stream(a.adj + k);
+      nd[q] = ld_stream(a.w + k);
     }
   }
-  if (LOCAL) queue_push(a, hub && mark(qbits(a, round + 1), v), v, o.QN, o.qnext, o.HV, o.HB, o.hnext);
-  int inc = d;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {  // dist of the rows: first needed here
+    const int dv = __shfl_sync(FULL, w.dv, j[q]);
+    const long long x = (long long)dv + nd[q];
+    nd[q] = t0 + 32 * q + lane < w.total && dv != INT_MAX && x < (long long)INT_MAX ? (int)x : INT_MAX;
+  }
+  relax_targets<LOCAL, N>(a, u, nd, thr, round, epoch, o, r);
+}
+
+// Relaxes the rows of the warp's lanes: lane i < n holds d >= 0 entries from b, of a vertex
+// at distance dv. An empty row takes one position that relaxes nothing, so that every lane
+// below n starts somewhere. Not LOCAL: improved vertices gather in the ring and go to the
+// next round's queue 32 at a time (a step improves a few of its 128 targets: marking and
+// queueing them step by step took one counter atomic and a pass of mostly idle lanes each).
+// LOCAL, rows of SU entries at most (a grid's): each lane takes its own row, without the
+// scan. `work` counts the edges relaxed.
+template <bool LOCAL>
+__device__ __forceinline__ void relax_rows(const Args& a, int n, int b, int d, int dv, int thr, int round, int epoch,
+                                           const Out& o, Ring& r, int& work) {
+  const int lane = threadIdx.x & 31;
+  if (!__any_sync(FULL, lane < n && d > 0)) return;
+  if (LOCAL && !__any_sync(FULL, lane < n && d > SU)) {
+    int u[SU], nd[SU];
+#pragma unroll
+    for (int q = 0; q < SU; ++q) {
+      u[q] = nd[q] = 0;
+      if (lane < n && q < d) {
+        u[q] = ld_stream(a.adj + b + q);
+        nd[q] = ld_stream(a.w + b + q);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < SU; ++q) {
+      const long long x = (long long)dv + nd[q];
+      nd[q] = lane < n && q < d && dv != INT_MAX && x < (long long)INT_MAX ? (int)x : INT_MAX;
+    }
+    work += __reduce_add_sync(FULL, lane < n ? d : 0);
+    relax_targets<LOCAL, SU>(a, u, nd, thr, round, epoch, o, r);
+    return;
+  }
+  const bool none = lane < n && d == 0;
+  int inc = lane < n ? (none ? 1 : d) : 0;
+  const int len = inc;
 #pragma unroll
   for (int k = 1; k < 32; k <<= 1) {
     const int t = __shfl_up_sync(FULL, inc, k);
     if (lane >= k) inc += t;
   }
-  const int total = __shfl_sync(FULL, inc, 31);
-  const int excl = inc - d;
-  work += total;
-  for (int t0 = 0; t0 < total; t0 += 32 * SU) {
-    int u[SU], res[SU], wt[SU], jq[SU];
-    long long nd[SU];
-#pragma unroll
-    for (int q = 0; q < SU; ++q) {
-      const int t = t0 + 32 * q + lane;
-      int j = 0;
-#pragma unroll
-      for (int k = 16; k > 0; k >>= 1)
-        if (__shfl_sync(FULL, excl, j + k) <= t) j += k;
-      const int jb = __shfl_sync(FULL, b, j);
-      const int je = __shfl_sync(FULL, excl, j);
-      jq[q] = j;
-      u[q] = 0;
-      wt[q] = 0;
-      if (t < total) {
-        const int k = jb + (t - je);
-        u[q] = ld_stream(a.adj + k);
-        wt[q] = ld_stream(a.w + k);
-      }
+  Rows w;
+  w.n = n;
+  w.total = __shfl_sync(FULL, inc, 31);
+  w.excl = inc - len;
+  w.shift = (none ? 0 : b) - w.excl;
+  w.dv = none ? INT_MAX : dv;
+  work += w.total - __popc(__ballot_sync(FULL, none));
+  int before = 0;
+  for (int t0 = 0; t0 < w.total;) {
+    if (w.total - t0 <= 32) {
+      relax_step<LOCAL, 1>(a, w, t0, before, thr, round, epoch, o, r);
+      t0 += 32;
+    } else {
+      relax_step<LOCAL, SU>(a, w, t0, before, thr, round, epoch, o, r);
+      t0 += 32 * SU;
     }
-#pragma unroll
-    for (int q = 0; q < SU; ++q) {
-      const long long jd = __shfl_sync(FULL, dv, jq[q]);
-      nd[q] = t0 + 32 * q + lane < total ? jd + wt[q] : (long long)INT_MAX;
-    }
-    relax_group<!LOCAL, SU>(a, u, nd, thr, round, epoch, o.fmin, res);
-    push_group<LOCAL, SU>(a, res, u, round, o, r);
+    if (!LOCAL)
+      while (r.cnt >= 32) ring_flush(a, round, o, r);
   }
 }
 
-// Edges [vb, ve) of one vertex at distance vd, 32 per step (a hub piece).
+// Relaxes the out-edges of a batch of the queue: lane i < n holds frontier vertex v.
 template <bool LOCAL>
-__device__ __forceinline__ void relax_range(const Args& a, int vb, int ve, long long vd, long long thr, int round,
-                                            int epoch, const Out& o, Ring& r) {
-  const int lane = threadIdx.x & 31;
-  for (int k0 = vb; k0 < ve; k0 += 32 * SU) {
-    int u[SU], res[SU];
-    long long nd[SU];
-#pragma unroll
-    for (int q = 0; q < SU; ++q) {
-      const int k = k0 + 32 * q + lane;
-      u[q] = 0;
-      nd[q] = INT_MAX;
-      if (k < ve) {
-        u[q] = ld_stream(a.adj + k);
-        nd[q] = vd + ld_stream(a.w + k);
-      }
-    }
-    relax_group<!LOCAL, SU>(a, u, nd, thr, round, epoch, o.fmin, res);
-    push_group<LOCAL, SU>(a, res, u, round, o, r);
+__device__ __forceinline__ void relax_batch(const Args& a, int v, int n, int thr, int round, int epoch, const Out& o,
+                                            Ring& r, int& work) {
+  int b = 0, d = 0, dv = INT_MAX;
+  if ((threadIdx.x & 31) < n) {
+    b = a.off[v];
+    const int e = a.off[v + 1];
+    dv = __ldcg(a.dist + v);
+    d = e - b;
   }
+  relax_rows<LOCAL>(a, n, b, d, dv, thr, round, epoch, o, r, work);
 }
 
 // Warp-local cascade: relax the ring, 32 entries at a time, until it is empty or the
 // warp has relaxed a.local_edges edges; what is left goes to the next round's queue.
 // Each pass either relaxes edges (work grows) or only pops, so the loop ends.
-__device__ __forceinline__ void cascade(const Args& a, long long thr, int round, int epoch, const Out& o, Ring& r,
+__device__ __forceinline__ void cascade(const Args& a, int thr, int round, int epoch, const Out& o, Ring& r,
                                         int& relaxed) {
   const int lane = threadIdx.x & 31;
   int work = 0;
   while (r.cnt > 0 && work < a.local_edges) {
     __syncwarp();
     const int take = min(r.cnt, 32);
-    const int v = lane < take ? r.s[(r.head + lane) & (RING - 1)] : -1;
+    int b = 0, d = 0, dv = INT_MAX;
+    if (lane < take) {
+      const int i = (r.head + lane) & (RING - 1);
+      dv = __ldcg(a.dist + r.s->v[i]);
+      b = r.s->b[i];
+      d = r.s->d[i];
+    }
     __syncwarp();
     r.head = (r.head + take) & (RING - 1);
     r.cnt -= take;
-    relax_batch<true>(a, v, thr, round, epoch, o, r, work);
+    relax_rows<true>(a, take, b, d, dv, thr, round, epoch, o, r, work);
   }
   relaxed += work;
-  __syncwarp();
-  for (int i0 = 0; i0 < r.cnt; i0 += 32) {
-    const int i = i0 + lane;
-    int u = 0;
-    bool want = false;
-    if (i < r.cnt) {
-      u = r.s[(r.head + i) & (RING - 1)];
-      want = mark(qbits(a, round + 1), u);
-    }
-    queue_push(a, want, u, o.QN, o.qnext, o.HV, o.HB, o.hnext);
-  }
-  __syncwarp();
-  r.head = 0;
-  r.cnt = 0;
+  while (r.cnt > 0) ring_flush(a, round, o, r);
 }
 
 // The inputs of the per-epoch width choice for candidate factor f (all from values
@@ -496,7 +538,13 @@ __device__ int epoch_choice(const Args& a, float fn, float rounds_prev, float re
 
 // One delta-stepping solve by `nblk` co-resident CTAs (this one is number `blk`):
 // the whole grid for a single source, or one group of a batched launch.
-__device__ __forceinline__ void delta_run(const Args& a, const int blk, const int nblk, int32_t* ring) {
+// What bounds it: the chain of dependent round trips of a step. With a search over lanes,
+// every step's marks, counters and far pushes waited for in the step, and rows loaded when
+// popped, a cascade step took 5,500 cycles for 25 to 35 edges on the grid, and an R-MAT
+// step issued one counter atomic and mostly idle passes per 128 edges. Now (rings, bit
+// windows, rows beside the atomicMins): grid 4096^2 31.5 -> 22.0 ms, R-MAT 23 6.98 -> 3.49
+// ms (13 rounds, 320 M edges relaxed), ER 2^20 2.2 -> 1.3 ms, grid 300^2 1.44 -> 1.10 ms.
+__device__ __forceinline__ void delta_run(const Args& a, const int blk, const int nblk, RingMem* ring) {
   Ctl* c = a.ctl;
   const int lane = threadIdx.x & 31;
   const int gw = (blk * THREADS + threadIdx.x) >> 5;
@@ -526,40 +574,54 @@ __device__ __forceinline__ void delta_run(const Args& a, const int blk, const in
       const Out o = {a.q[(round + 1) & 1], &c->qcount[(round + 1) % 3], a.hv[(round + 1) & 1],
                      a.hbase[(round + 1) & 1], &c->hcount[(round + 1) % 3], a.f[epoch & 1], &c->fcount[epoch % 3],
                      &c->fmin[epoch % 3]};
-      Ring r = {ring + (threadIdx.x >> 5) * RING, 0, 0};
+      Ring r = {ring + (threadIdx.x >> 5), 0, 0, 0, 0, INT_MAX};
       // a small frontier is spread over all warps (fewer entries per warp, fewer steps)
       const int per = min(32, max(1, (qn + nw - 1) / nw));
       const bool local = a.local_edges > 0 && qn <= nw * 32;
+      const int t32 = (int)min(thr, (long long)INT_MAX);  // every distance is below INT_MAX
       int work = 0;
       for (int base = gw * per; base < qn; base += nw * per) {
-        const int v = (lane < per && base + lane < qn) ? Q[base + lane] : -1;
+        const int n = min(per, qn - base);
+        const int v = lane < n ? Q[base + lane] : -1;
         if (local)
-          relax_batch<true>(a, v, thr, round, epoch, o, r, work);
+          relax_batch<true>(a, v, n, t32, round, epoch, o, r, work);
         else
-          relax_batch<false>(a, v, thr, round, epoch, o, r, work);
+          relax_batch<false>(a, v, n, t32, round, epoch, o, r, work);
       }
-      // hub pieces of this round: hub_chunk edges per warp, all warps
-      {
+      // hub pieces of this round: runs of consecutive pieces dealt to the warps in turn, up to
+      // 32 a run. A run's first hub is searched for; its hubs follow in the list.
+      if (hchunks > 0) {
         const int32_t* HVc = a.hv[round & 1];
         const int32_t* HBc = a.hbase[round & 1];
-        for (int ch = gw; ch < hchunks; ch += nw) {
-          int lo = 0, hi = hn - 1;  // last entry whose first chunk <= ch
+        const int run = min(HUB_RUN, (hchunks + nw - 1) / nw);
+        for (long long c = (long long)gw * run; c < hchunks; c += (long long)nw * run) {
+          const int c0 = (int)c, c1 = (int)min(c + run, (long long)hchunks);
+          int lo = 0, hi = hn - 1;  // last entry whose first piece <= c0
           while (lo < hi) {
             const int m = (lo + hi + 1) >> 1;
-            if (HBc[m] <= ch) lo = m; else hi = m - 1;
+            if (HBc[m] <= c0) lo = m; else hi = m - 1;
           }
-          const int v = HVc[lo];
-          const long long vd = __ldcg(a.dist + v);
-          const int vb = a.off[v] + (ch - HBc[lo]) * a.hub_chunk;
-          const int ve = min(vb + a.hub_chunk, a.off[v + 1]);
-          work += max(0, ve - vb);
+          const int first = lo + lane < hn ? HBc[lo + lane] : INT_MAX;
+          int b = 0, d = 0, dv = INT_MAX;
+          if (first < c1) {
+            const int v = HVc[lo + lane];
+            dv = __ldcg(a.dist + v);
+            const int vb = a.off[v], ve = a.off[v + 1];
+            b = vb + max(0, c0 - first) * a.hub_chunk;
+            d = (int)min((long long)ve, vb + (long long)(c1 - first) * a.hub_chunk) - b;
+          }
+          const int n = __popc(__ballot_sync(FULL, first < c1));
           if (local)
-            relax_range<true>(a, vb, ve, vd, thr, round, epoch, o, r);
+            relax_rows<true>(a, n, b, d, dv, t32, round, epoch, o, r, work);
           else
-            relax_range<false>(a, vb, ve, vd, thr, round, epoch, o, r);
+            relax_rows<false>(a, n, b, d, dv, t32, round, epoch, o, r, work);
         }
       }
-      if (local) cascade(a, thr, round, epoch, o, r, work);
+      if (local) cascade(a, t32, round, epoch, o, r, work);
+      while (r.cnt > 0) ring_flush(a, round, o, r);
+      while (r.fcnt > 0) far_flush(a, epoch, o, r);
+      const int fm = __reduce_min_sync(FULL, r.fmin);
+      if (lane == 0 && fm != INT_MAX) atomicMin(o.fmin, fm);
       if (lane == 0 && work > 0) atomicAdd(&c->relaxed, (unsigned long long)work);
       if (blk == 0 && threadIdx.x == 0) {
         c->qcount[(round + 2) % 3] = 0;  // read two rounds ago
@@ -662,7 +724,7 @@ __device__ __forceinline__ void delta_run(const Args& a, const int blk, const in
 }
 
 __global__ void __launch_bounds__(THREADS, 4) k_delta(Args a) {
-  __shared__ int32_t ring[(THREADS / 32) * RING];
+  __shared__ RingMem ring[THREADS / 32];
   delta_run(a, blockIdx.x, gridDim.x, ring);
 }
 
@@ -671,7 +733,7 @@ __global__ void __launch_bounds__(THREADS, 4) k_delta(Args a) {
 // and its own Ctl (counters, bounded group barrier). Adjacency, weights and offsets
 // are shared, so the groups' gathers share L2.
 __global__ void __launch_bounds__(THREADS, 4) k_delta_multi(Args a, int gsz) {
-  __shared__ int32_t ring[(THREADS / 32) * RING];
+  __shared__ RingMem ring[THREADS / 32];
   __shared__ Args b;  // this group's arguments (shared: read like the kernel parameters)
   const int g = blockIdx.x / gsz;
   if (threadIdx.x == 0) {
