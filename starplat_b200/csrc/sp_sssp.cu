@@ -46,6 +46,10 @@ namespace sp {
 
 namespace ss {
 constexpr int THREADS = 256;
+// Resident CTAs an SM the kernels are compiled for (the schedule runs as many or fewer). R-MAT
+// 23 / ER 2^20 / grid 4096^2: 3.69 / 1.31 / 17.0 ms at 4 (64 registers, spills), 3.58 / 1.11 /
+// 16.8 at 3, 4.76 / 0.97 / 17.2 at 2.
+constexpr int CTAS = 3;
 // Queued vertices above HUB_DEG out-edges are relaxed in HUB_CHUNK-edge pieces that
 // every warp shares, so no warp walks a long row alone while the others wait at the
 // round's barrier. A warp takes up to HUB_RUN consecutive pieces as the rows of one batch
@@ -59,12 +63,13 @@ constexpr int HUB_DEG_MAX = 1 << 25;  // 32 entries of at most this degree sum b
 constexpr int RING = 256;             // entries of a warp's rings (a power of two above 31 + 32 * SU)
 constexpr int LOCAL_STEPS = 64;       // default cascade budget: 32-edge warp steps per round
 constexpr int SU = 4;                 // 32-edge windows whose loads and atomics are in flight together
-// Sources per cooperative launch of the batched form. 16 weighted closeness sources of
-// undirected R-MAT 20: 34.1 ms with 1 per launch, 34.5 with 4 or 8, 36.0 with 16.
-constexpr int BATCH = 4;
+// Sources per cooperative launch of the batched form. 16 sources of undirected R-MAT 20 /
+// grid 1024^2: 17.2 / 58.8 ms with 1 per launch, 12.5 / 17.5 with 4, 11.4 / 10.3 with 8,
+// 11.5 / 7.9 with 16 (each needs nine V-sized buffers).
+constexpr int BATCH = 8;
 // sp_sssp_dynamic repairs a batch with deletions by default when the graph's last solve
-// took at least this many rounds (grid 1024^2 repairs in 1.5 ms against 8.3 ms for a new
-// solve; R-MAT 20, a dozen rounds, 3.4 against 2.2 ms).
+// took at least this many rounds (100 deletions, the update included: grid 1024^2 repairs in
+// 3.7 ms against 5.3 for a new solve; R-MAT 20, a dozen rounds, 7.9 against 3.9).
 constexpr int REPAIR_MIN_ROUNDS = 32;
 constexpr unsigned FULL = 0xffffffffu;
 
@@ -198,12 +203,11 @@ __device__ __forceinline__ void warp_push(const Args& a, bool want, int val, int
 
 // Queue u for the next round: hubs go to the hub list (with their chunk count),
 // everything else to the near queue (warp-aggregated).
-__device__ __forceinline__ void queue_push(const Args& a, bool want, int u, int32_t* QN, int* qnext, int32_t* HV,
+__device__ __forceinline__ void queue_push(const Args& a, bool want, int u, int d, int32_t* QN, int* qnext, int32_t* HV,
                                            int32_t* HB, unsigned long long* hcnt) {
   bool hub = false;
   int nch = 0;
   if (want) {
-    const int d = a.off[u + 1] - a.off[u];
     if (d > a.hub_deg) {
       hub = true;
       nch = (d + a.hub_chunk - 1) / a.hub_chunk;
@@ -267,7 +271,7 @@ __device__ __forceinline__ void ring_push(const Args& a, const bool (&near)[N], 
     }
     r.cnt += min(__popc(m[q]), room);
     const bool rest = near[q] && !mine && mark(qbits(a, round + 1), u[q]);
-    queue_push(a, rest, u[q], o.QN, o.qnext, o.HV, o.HB, o.hnext);
+    queue_push(a, rest, u[q], d[q], o.QN, o.qnext, o.HV, o.HB, o.hnext);
   }
 }
 
@@ -277,13 +281,14 @@ __device__ __forceinline__ void ring_flush(const Args& a, int round, const Out& 
   const int lane = threadIdx.x & 31;
   __syncwarp();
   const int take = min(r.cnt, 32);
-  int u = 0;
+  int u = 0, d = 0;
   bool want = false;
   if (lane < take) {
     u = r.s->v[(r.head + lane) & (RING - 1)];
+    d = a.off[u + 1] - a.off[u];
     want = mark(qbits(a, round + 1), u);
   }
-  queue_push(a, want, u, o.QN, o.qnext, o.HV, o.HB, o.hnext);
+  queue_push(a, want, u, d, o.QN, o.qnext, o.HV, o.HB, o.hnext);
   __syncwarp();
   r.head = (r.head + take) & (RING - 1);
   r.cnt -= take;
@@ -363,6 +368,12 @@ __device__ __forceinline__ void relax_targets(const Args& a, const int (&u)[N], 
   }
 }
 
+// dist + weight; INT_MAX (no distance) from an unreached vertex or past INT_MAX.
+__device__ __forceinline__ int candidate(int dv, int wt) {
+  const int x = (int)((unsigned)dv + (unsigned)wt);
+  return dv == INT_MAX || (wt > 0 && x < dv) ? INT_MAX : x;
+}
+
 // A warp's rows: lane i < n holds the row of d entries from b at distance dv. Lane i's
 // entries take positions [excl, excl + d) of the flattened rows.
 struct Rows {
@@ -399,8 +410,7 @@ __device__ __forceinline__ void relax_step(const Args& a, const Rows& w, int t0,
 #pragma unroll
   for (int q = 0; q < N; ++q) {  // dist of the rows: first needed here
     const int dv = __shfl_sync(FULL, w.dv, j[q]);
-    const long long x = (long long)dv + nd[q];
-    nd[q] = t0 + 32 * q + lane < w.total && dv != INT_MAX && x < (long long)INT_MAX ? (int)x : INT_MAX;
+    nd[q] = t0 + 32 * q + lane < w.total ? candidate(dv, nd[q]) : INT_MAX;
   }
   relax_targets<LOCAL, N>(a, u, nd, thr, round, epoch, o, r);
 }
@@ -410,32 +420,12 @@ __device__ __forceinline__ void relax_step(const Args& a, const Rows& w, int t0,
 // below n starts somewhere. Not LOCAL: improved vertices gather in the ring and go to the
 // next round's queue 32 at a time (a step improves a few of its 128 targets: marking and
 // queueing them step by step took one counter atomic and a pass of mostly idle lanes each).
-// LOCAL, rows of SU entries at most (a grid's): each lane takes its own row, without the
-// scan. `work` counts the edges relaxed.
+// `work` counts the edges relaxed.
 template <bool LOCAL>
 __device__ __forceinline__ void relax_rows(const Args& a, int n, int b, int d, int dv, int thr, int round, int epoch,
                                            const Out& o, Ring& r, int& work) {
   const int lane = threadIdx.x & 31;
   if (!__any_sync(FULL, lane < n && d > 0)) return;
-  if (LOCAL && !__any_sync(FULL, lane < n && d > SU)) {
-    int u[SU], nd[SU];
-#pragma unroll
-    for (int q = 0; q < SU; ++q) {
-      u[q] = nd[q] = 0;
-      if (lane < n && q < d) {
-        u[q] = ld_stream(a.adj + b + q);
-        nd[q] = ld_stream(a.w + b + q);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < SU; ++q) {
-      const long long x = (long long)dv + nd[q];
-      nd[q] = lane < n && q < d && dv != INT_MAX && x < (long long)INT_MAX ? (int)x : INT_MAX;
-    }
-    work += __reduce_add_sync(FULL, lane < n ? d : 0);
-    relax_targets<LOCAL, SU>(a, u, nd, thr, round, epoch, o, r);
-    return;
-  }
   const bool none = lane < n && d == 0;
   int inc = lane < n ? (none ? 1 : d) : 0;
   const int len = inc;
@@ -479,6 +469,49 @@ __device__ __forceinline__ void relax_batch(const Args& a, int v, int n, int thr
   relax_rows<LOCAL>(a, n, b, d, dv, thr, round, epoch, o, r, work);
 }
 
+// The ring's oldest `take` entries (at most 8 * N), four lanes to a row, so that rows of up
+// to four entries (a grid's) need no scan and no owner search; false (and nothing done)
+// when one is longer. Grid 4096^2: 20.4 -> 17.0 ms (a lane to a row: four loads and four
+// atomics a lane however few rows there are), 21.3 with 16 rows a step at most.
+template <int N>
+__device__ __forceinline__ bool cascade_quads(const Args& a, int take, int thr, int round, int epoch, const Out& o,
+                                              Ring& r, int& work) {
+  const int lane = threadIdx.x & 31, col = lane & 3;
+  int b[N], d[N], dv[N], u[N], nd[N];
+  bool lng = false;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    const int row = 8 * q + (lane >> 2), i = (r.head + row) & (RING - 1);
+    b[q] = d[q] = dv[q] = 0;
+    if (row < take) {
+      u[q] = r.s->v[i];
+      b[q] = r.s->b[i];
+      d[q] = r.s->d[i];
+    }
+    lng |= d[q] > 4;
+  }
+  if (__any_sync(FULL, lng)) return false;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    const bool on = col < d[q];
+    work += __popc(__ballot_sync(FULL, on));
+    if (on) {
+      dv[q] = __ldcg(a.dist + u[q]);
+      u[q] = ld_stream(a.adj + b[q] + col);
+      nd[q] = ld_stream(a.w + b[q] + col);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    nd[q] = col < d[q] ? candidate(dv[q], nd[q]) : INT_MAX;
+  }
+  r.head = (r.head + take) & (RING - 1);
+  r.cnt -= take;
+  __syncwarp();
+  relax_targets<true, N>(a, u, nd, thr, round, epoch, o, r);
+  return true;
+}
+
 // Warp-local cascade: relax the ring, 32 entries at a time, until it is empty or the
 // warp has relaxed a.local_edges edges; what is left goes to the next round's queue.
 // Each pass either relaxes edges (work grows) or only pops, so the loop ends.
@@ -489,6 +522,10 @@ __device__ __forceinline__ void cascade(const Args& a, int thr, int round, int e
   while (r.cnt > 0 && work < a.local_edges) {
     __syncwarp();
     const int take = min(r.cnt, 32);
+    if (take <= 8    ? cascade_quads<1>(a, take, thr, round, epoch, o, r, work)
+        : take <= 16 ? cascade_quads<2>(a, take, thr, round, epoch, o, r, work)
+                     : cascade_quads<4>(a, take, thr, round, epoch, o, r, work))
+      continue;
     int b = 0, d = 0, dv = INT_MAX;
     if (lane < take) {
       const int i = (r.head + lane) & (RING - 1);
@@ -542,8 +579,9 @@ __device__ int epoch_choice(const Args& a, float fn, float rounds_prev, float re
 // every step's marks, counters and far pushes waited for in the step, and rows loaded when
 // popped, a cascade step took 5,500 cycles for 25 to 35 edges on the grid, and an R-MAT
 // step issued one counter atomic and mostly idle passes per 128 edges. Now (rings, bit
-// windows, rows beside the atomicMins): grid 4096^2 31.5 -> 22.0 ms, R-MAT 23 6.98 -> 3.49
-// ms (13 rounds, 320 M edges relaxed), ER 2^20 2.2 -> 1.3 ms, grid 300^2 1.44 -> 1.10 ms.
+// windows, rows beside the atomicMins, four lanes to a row): grid 4096^2 28.9 -> 16.8 ms,
+// R-MAT 23 6.98 -> 3.58 ms (13 rounds, 330 M edges relaxed), ER 2^20 2.2 -> 1.1 ms, grid
+// 300^2 1.44 -> 0.93 ms.
 __device__ __forceinline__ void delta_run(const Args& a, const int blk, const int nblk, RingMem* ring) {
   Ctl* c = a.ctl;
   const int lane = threadIdx.x & 31;
@@ -697,7 +735,7 @@ __device__ __forceinline__ void delta_run(const Args& a, const int blk, const in
             }
           }
         }
-        queue_push(a, toq, u, Q, qcnt, HV, HB, hnext);
+        queue_push(a, toq, u, toq ? a.off[u + 1] - a.off[u] : 0, Q, qcnt, HV, HB, hnext);
         warp_push(a, tof, u, FN, fnext);
       }
       if (blk == 0 && threadIdx.x == 0) {
@@ -723,7 +761,7 @@ __device__ __forceinline__ void delta_run(const Args& a, const int blk, const in
   }
 }
 
-__global__ void __launch_bounds__(THREADS, 4) k_delta(Args a) {
+__global__ void __launch_bounds__(THREADS, CTAS) k_delta(Args a) {
   __shared__ RingMem ring[THREADS / 32];
   delta_run(a, blockIdx.x, gridDim.x, ring);
 }
@@ -732,7 +770,7 @@ __global__ void __launch_bounds__(THREADS, 4) k_delta(Args a) {
 // g-th source of the batch over its own V-strided slice of every per-vertex buffer
 // and its own Ctl (counters, bounded group barrier). Adjacency, weights and offsets
 // are shared, so the groups' gathers share L2.
-__global__ void __launch_bounds__(THREADS, 4) k_delta_multi(Args a, int gsz) {
+__global__ void __launch_bounds__(THREADS, CTAS) k_delta_multi(Args a, int gsz) {
   __shared__ RingMem ring[THREADS / 32];
   __shared__ Args b;  // this group's arguments (shared: read like the kernel parameters)
   const int g = blockIdx.x / gsz;
