@@ -62,3 +62,33 @@ def test_fixed_iterations_match_the_oracle(name):
         none = (np.empty(0, "S1"), np.empty(0, np.int32), np.empty(0, np.int32), None)
         warm, _, _ = dg.pagerank_dynamic(*none, part, 0.0, 0.85, 17)
         assert np.abs(warm.astype(np.float64) - ref).sum() < 1e-6
+
+
+@pytest.mark.parametrize("iters", [15, 16, 17, 24, 25, 60])
+def test_first_call_stops_at_the_iteration_it_would(iters):
+    # above the one-launch sizes a first call reads the stop test after 16, 24, 36 ...
+    # iterations, a second launches them all: the same ranks, count and change
+    g = GRAPHS["er_above"]() if iters == 60 else GRAPHS["hubs_above"]()
+    with DeviceGraph.from_csr(g, with_weights=False) as dg:
+        first = dg.pagerank(1e-6 if iters == 60 else 0.0, 0.85, iters)
+        again = dg.pagerank(1e-6 if iters == 60 else 0.0, 0.85, iters)
+        assert first[1] == again[1] and (iters == 60 or first[1] == iters)
+        # the change is a sum over CTAs in one order, so it and the ranks are the same bits
+        assert first[2] == again[2] and np.array_equal(first[0], again[0])
+
+
+@pytest.mark.parametrize("order", [0, 1])
+def test_transpose_of_rows_of_every_length(order):
+    # rows of 0 to 4 entries, around a window (32), a warp's row (128) and a CTA's (1,024)
+    rng = np.random.default_rng(3)
+    degrees = np.concatenate([np.tile([0, 1, 2, 4, 31, 32, 33], 40), [127, 128, 129, 130, 1023, 1024, 1025, 3000]])
+    V = 4000
+    src = np.repeat(np.arange(len(degrees)), degrees)
+    dst = np.concatenate([rng.choice(V, d, replace=False) for d in degrees])
+    g = from_pairs(V, np.stack([src, dst], 1))
+    g.ensure_reverse()
+    with DeviceGraph.from_csr(g, with_weights=False) as dg:
+        dg.tune_set("pr.order", order)
+        out, _, _ = dg.pagerank(0.0, 0.85, 3)
+    ref, _, _ = O.pagerank(g.indexofNodes, g.rev_indexofNodes, g.srcList, 0.0, 0.85, 3, fixed_iters=3)
+    assert np.abs(out.astype(np.float64) - ref).sum() < 1e-6
