@@ -47,7 +47,7 @@ struct Block {
 };
 struct BlockCache {
   std::mutex mu;
-  std::vector<Block> blocks;
+  std::vector<Block> blocks;  // oldest first
   size_t cached[64] = {};  // bytes held per device
   size_t cap[64] = {};     // at most min(1/8 of the device's memory, 4 GiB) is held
 };
@@ -75,8 +75,7 @@ size_t drain(int dev) {
     if (b.device != cur) cudaSetDevice(cur);
     c.cached[b.device] -= b.bytes;
     freed += b.bytes;
-    c.blocks[i] = c.blocks.back();
-    c.blocks.pop_back();
+    c.blocks.erase(c.blocks.begin() + i);
   }
   return freed;
 }
@@ -98,8 +97,7 @@ int dev_alloc(void** p, size_t bytes, size_t* got, int* dev) {
     }
     if (best >= 0) {
       const Block b = c.blocks[best];
-      c.blocks[best] = c.blocks.back();
-      c.blocks.pop_back();
+      c.blocks.erase(c.blocks.begin() + best);
       c.cached[d] -= b.bytes;
       *p = b.p;
       *got = b.bytes;
@@ -143,9 +141,22 @@ void dev_free(void* p, size_t bytes, int dev) {
     // other allocators in the process (torch's) cannot reclaim what this cache holds
     c.cap[dev] = cudaMemGetInfo(&fr, &tot) == cudaSuccess ? std::min(tot / 8, (size_t)4 << 30) : 0;
   }
-  if (c.cached[dev] + bytes > c.cap[dev]) {
+  if (bytes > c.cap[dev]) {
     cudaFree(p);
     return;
+  }
+  // A full cache gives up its oldest blocks for the new one. While it turned the new one
+  // away instead, blocks left by a larger graph stayed for good and every call of a smaller
+  // one paid cudaMalloc and cudaFree: a batch of updates with ranks on R-MAT 20 after
+  // PageRank on R-MAT 22 in the same process 9 to 24 ms a call, now 5.1 (alone 5.1).
+  for (size_t i = 0; i < c.blocks.size() && c.cached[dev] + bytes > c.cap[dev];) {
+    if (c.blocks[i].device != dev) {
+      ++i;
+      continue;
+    }
+    cudaFree(c.blocks[i].p);
+    c.cached[dev] -= c.blocks[i].bytes;
+    c.blocks.erase(c.blocks.begin() + i);
   }
   c.blocks.push_back({p, bytes, dev});
   c.cached[dev] += bytes;
