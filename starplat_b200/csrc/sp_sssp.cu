@@ -169,6 +169,15 @@ __device__ __forceinline__ int ld_stream(const int32_t* p) {
   return v;
 }
 
+// The filter's view of a distance may be an older one from L1: distances only fall during a
+// solve, so an older value is a larger one and lets a candidate through that the atomicMin
+// then turns down. Reading past L1, R-MAT 20 0.77 ms, now 0.71; R-MAT 23 3.58 and 3.54.
+__device__ __forceinline__ int ld_filter(const int32_t* p) {
+  int v;
+  asm volatile("ld.global.ca.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // Sets vertex u's bit in bm; true for the one caller that set it first.
 __device__ __forceinline__ bool mark(unsigned* bm, int u) {
   const unsigned b = 1u << (u & 31);
@@ -330,7 +339,7 @@ __device__ __forceinline__ void relax_targets(const Args& a, const int (&u)[N], 
 #pragma unroll
   for (int q = 0; q < N; ++q) {
     old[q] = INT_MAX;
-    if (filt && nd[q] != INT_MAX) old[q] = __ldcg(a.dist + u[q]);
+    if (filt && nd[q] != INT_MAX) old[q] = ld_filter(a.dist + u[q]);
   }
 #pragma unroll
   for (int q = 0; q < N; ++q) {
@@ -1526,7 +1535,7 @@ extern "C" int sp_sssp_dynamic(sp_graph_h g, int64_t n, const char* type, const 
   bool repair = false;
   g->sssp_last_marked = -1;
   // By default the repair runs on graphs whose last solve from a source took at least
-  // REPAIR_MIN_ROUNDS rounds: where a solve takes a dozen rounds (R-MAT 20: 1.3 ms) its
+  // REPAIR_MIN_ROUNDS rounds: where a solve takes a dozen rounds (R-MAT 20: 0.8 ms) its
   // fixed passes over the graph cost more than solving again.
   const bool want_repair = g->sssp_repair > 0 || (g->sssp_repair < 0 && g->sssp_last_rounds >= ss::REPAIR_MIN_ROUNDS);
   if (deletes && want_repair) {
