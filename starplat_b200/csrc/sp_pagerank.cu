@@ -170,12 +170,14 @@ struct IterArgs {
   double* diff_out;  // split plan: this part's L1 diff of the iteration (summed over parts by the caller)
 };
 
+// LIVE: pr_old changes during the launch (k_run), so it is not read through the read-only path.
+template <bool LIVE>
 __device__ __forceinline__ double finalize_row(const IterArgs& a, int r, double sum,
                                                const float* __restrict__ pr_old, float* __restrict__ pr_new,
                                                float* __restrict__ con_new) {
   const float s = (float)sum;
   const float np = __fadd_rn(a.base, __fmul_rn(a.delta, s));
-  const float po = __ldcg(pr_old + r);
+  const float po = LIVE ? __ldcg(pr_old + r) : pr_old[r];
   pr_new[r] = np;
   const int od = a.od[r];
   con_new[r] = od > 0 ? __fdiv_rn(np, (float)od) : 0.0f;
@@ -230,6 +232,7 @@ __device__ __forceinline__ int comp4(const int4& q, int j) { return j == 0 ? q.x
 template <int SH, int GH>
 struct GatherGlobal {
   static constexpr int kSrcHint = SH;
+  static constexpr bool kLive = false;
   const float* __restrict__ con;
   int hot;
   __device__ __forceinline__ float operator()(int u) const {
@@ -246,6 +249,7 @@ struct GatherGlobal {
 template <int SH, int GH>
 struct GatherLive {
   static constexpr int kSrcHint = SH;
+  static constexpr bool kLive = true;
   const float* con;
   int hot;
   __device__ __forceinline__ float operator()(int u) const {
@@ -341,10 +345,10 @@ __device__ __forceinline__ double warp_task(const IterArgs& a, int start, int co
       a.part[r] = sum;
       return 0.0;
     }
-    return finalize_row(a, r, sum, pr_old, pr_new, con_new);
+    return finalize_row<G::kLive>(a, r, sum, pr_old, pr_new, con_new);
   }
   if (other > 0) sum += a.part[r];
-  return finalize_row(a, r, sum, pr_old, pr_new, con_new);
+  return finalize_row<G::kLive>(a, r, sum, pr_old, pr_new, con_new);
 }
 
 // The rows of one phase of one iteration by persistent CTAs of NT threads: long-row
@@ -417,7 +421,7 @@ __device__ __forceinline__ double phase_work(const IterArgs& a, const G& gather,
       double sum = 0;
       const volatile double* cp = a.chunk_part;
       for (int k = 0; k < L.y; ++k) sum += cp[L.x + k];
-      my_diff += finalize_row(a, c.x, sum, pr_old, pr_new, con_new);
+      my_diff += finalize_row<G::kLive>(a, c.x, sum, pr_old, pr_new, con_new);
       a.long_ctr[li] = 0;
     }
     __syncthreads();
