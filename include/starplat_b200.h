@@ -121,9 +121,10 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "sssp.delta"  SSSP bucket width used when sp_sssp gets delta <= 0 (0 = the largest
  *             edge weight).
  *   "sssp.ctas_per_sm"  SSSP: persistent CTAs per SM of the delta-stepping kernel (1..8,
- *             default 4; fewer CTAs make each grid barrier cheaper on high-diameter graphs).
+ *             default 4; at most the 3 that are resident run; fewer make each grid barrier
+ *             cheaper on high-diameter graphs).
  *   "sssp.batch"  sp_sssp_batch / sp_closeness: sources per cooperative launch, each on
- *             its own group of CTAs (1..1024, default 4; capped by the co-resident CTAs
+ *             its own group of CTAs (1..1024, default 8; capped by the co-resident CTAs
  *             and by 1/8 of device memory at 44 bytes per vertex per source).
  *   "sssp.last_batch" (read only): sources per launch of the last batched run.
  *   "sssp.last_delta", "sssp.last_ctas", "sssp.last_local" (read only): the schedule the
@@ -131,6 +132,8 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *             out-edge of a vertex once per time the vertex was expanded).
  *   "tc.cta_warps"  TC on graphs of up to 65536 vertices: 0 = a bitmap per warp;
  *             2, 4, 8 or 16 = one bitmap per CTA of that many warps sharing each anchor.
+ *             At the default (4) symmetric graphs are counted in rank order instead (the
+ *             count itself from 65536 vertices or 131072 entries on).
  *   "tc.last_incremental" (read only): 1 if the last sp_tc_dynamic counted only the
  *             triangles through the batch's edges, 0 if it counted the graph again.
  *   "sssp.hub_deg", "sssp.hub_chunk"  SSSP: queued vertices with more out-edges than
@@ -139,9 +142,9 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "sssp.repair"  sp_sssp_dynamic: 1 = a batch with deletions repairs through parents
  *             (weights >= 1), 0 = it solves again from the source, -1 (default) = repair
  *             when the graph's last solve from a source took at least 32 rounds. The
- *             repair pays on high-diameter graphs (grid 1024^2, 64 deletions: 1.5 ms
- *             against 8.3 ms for update + solve) and loses where a solve takes a dozen
- *             rounds (R-MAT 20: 3.4 against 2.2 ms). "sssp.last_marked" (read only):
+ *             repair pays on high-diameter graphs (grid 1024^2, 100 deletions: 3.7 ms
+ *             against 5.3 ms for update + solve) and loses where a solve takes a dozen
+ *             rounds (R-MAT 20: 7.9 against 3.9 ms). "sssp.last_marked" (read only):
  *             vertices the last repair reset (-1: no repair ran).
  *   "sssp.filter"  SSSP: 1 = load dist[u] and send the atomicMin only when the candidate
  *             is lower; 0 = send every atomicMin at once (one L2 round trip less per
@@ -149,13 +152,14 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "sssp.local"  SSSP: in rounds whose frontier is at most 32 vertices per warp, a warp
  *             keeps relaxing the vertices it improved below the bucket threshold, up to
  *             this many 32-edge steps per round, before the grid barrier (0 = off,
- *             default 64). Unset, the learned scheduler chooses between 0 and 64.
+ *             default 64). Unset, the learned scheduler chooses 0, 64 or 256.
  *   "bc.hub_deg", "bc.hub_chunk"  BC: level-list entries of vertices with more than
  *             hub_deg edges are cut into hub_chunk-edge pieces shared by all warps
  *             (defaults 64 and 64).
  *   "bc.batch"  BC: sources traversed together in one multi-source pass (1..64, default 64).
  *   "bc.dir"  BC forward direction per level (one cooperative launch, sp_bc and
- *             sp_bfs_sigma): 0 push (expand the level's entries along out-edges);
+ *             sp_bfs_sigma): 0 the gathering form (an entry expands its level and sums its
+ *             own path counts); the others run the push / pull form:
  *             1 pull while bc.pull_alpha * (out-edges of the level's entries) exceeds the
  *             in-edges of the vertices some source has not reached + V / 8 (pull: every
  *             such vertex scans its in-edges for parents in the level, no atomics except
@@ -168,9 +172,9 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "bc.pull_alpha"  factor of the bc.dir = 1 rule, in thousandths (default 1000).
  *   "bc.trace"  1: record per level (entries, their out-edges, unreached in-edges, pull)
  *             and the device timer; read with sp_bc_level_trace.
- *   "bc.cluster"  BC of many graphs (sp_bc_graphs): CTAs per graph, 1 (default), 2, 4 or 8;
- *             above 1 the CTAs of a thread-block cluster share a graph and synchronise with
- *             hardware cluster barriers. */
+ *   "bc.cluster"  BC of many graphs (sp_bc_graphs): unset, all graphs run as one; set, CTAs
+ *             per graph, 1, 2, 4 or 8; above 1 the CTAs of a thread-block cluster share a graph
+ *             and synchronise with hardware cluster barriers. */
 int sp_tune_set(sp_graph_h g, const char* key, int64_t value);
 int sp_tune_get(sp_graph_h g, const char* key, int64_t* value);
 
