@@ -155,7 +155,8 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *             default 64). Unset, the learned scheduler chooses 0, 64 or 256.
  *   "bc.hub_deg", "bc.hub_chunk"  BC: level-list entries of vertices with more than
  *             hub_deg edges are cut into hub_chunk-edge pieces shared by all warps
- *             (defaults 64 and 64).
+ *             (defaults 64 and 64; 256 and 128 in the gathering form from 12 M entries on,
+ *             where neither is set).
  *   "bc.batch"  BC: sources traversed together in one multi-source pass (1..64, default 64).
  *   "bc.dir"  BC forward direction per level (one cooperative launch, sp_bc and
  *             sp_bfs_sigma): 0 the gathering form (an entry expands its level and sums its

@@ -50,6 +50,12 @@ constexpr int CTA_THREADS = 512;
 // 121 at (128, 256), 110 at (64, 64).
 constexpr int HUB_DEG = 64;
 constexpr int HUB_CHUNK = 64;
+// The gathering form on graphs of WIDE_E entries and more: fewer, longer pieces, as a level
+// then has entries enough to fill the warps, and pieces meet in an FP64 scratch. 64 sources of
+// undirected R-MAT at (64, 64) and (256, 128): scale 20 (31 M entries) 7.00 and 6.67 ms, 19
+// (15 M) 3.79 and 3.66, 18 (8 M) 2.11 and 2.23, 16 0.80 and 1.02; ER 2^19 (17 M) 5.75 both.
+constexpr int WIDE_HUB_DEG = 256, WIDE_HUB_CHUNK = 128;
+constexpr double WIDE_E = 12e6;
 constexpr int CLUSTER_DEFAULT = 1;  // CTAs per graph in the many-graphs form (bc.cluster)
 // Successors whose loads are in flight together in the backward sweep (measured when
 // each successor cost a sigma and a delta load),
@@ -1103,10 +1109,12 @@ static int bc_variant_pick(sp_graph* g, int nsrc, int* cand) {
   return SP_OK;
 }
 
-// bc.hub_deg / bc.hub_chunk of a call: the knobs, the learned variant, or the defaults.
-static int bc_split(sp_graph* g, int nsrc, int* hub_deg, int* hub_chunk) {
-  *hub_deg = g->bc_hub_deg > 0 ? g->bc_hub_deg : bc::HUB_DEG;
-  *hub_chunk = g->bc_hub_chunk > 0 ? g->bc_hub_chunk : bc::HUB_CHUNK;
+// bc.hub_deg / bc.hub_chunk of a call: the knobs, the learned variant, or the defaults
+// (wide: those of the gathering form on large graphs, where neither knob is set).
+static int bc_split(sp_graph* g, int nsrc, int* hub_deg, int* hub_chunk, bool wide = false) {
+  wide = wide && g->bc_hub_deg <= 0 && g->bc_hub_chunk <= 0;
+  *hub_deg = g->bc_hub_deg > 0 ? g->bc_hub_deg : wide ? bc::WIDE_HUB_DEG : bc::HUB_DEG;
+  *hub_chunk = g->bc_hub_chunk > 0 ? g->bc_hub_chunk : wide ? bc::WIDE_HUB_CHUNK : bc::HUB_CHUNK;
   int cand = -1;
   SP_TRY(bc_variant_pick(g, nsrc, &cand));
   if (cand >= 0) {
@@ -1139,7 +1147,7 @@ static int bc_gather(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch, in
   const size_t cap = (size_t)V * std::min(width, 16) + 1024;  // level-list entries (vertex, mask)
   bc::GatherArgs a;
   bc::Gather& W = a.G;
-  SP_TRY(bc_split(g, nsrc, &W.hub_deg, &W.hub_chunk));
+  SP_TRY(bc_split(g, nsrc, &W.hub_deg, &W.hub_chunk, (double)g->E >= bc::WIDE_E));
   // Pieces of one pass over the graph: at most E / chunk + E / hub_deg. A vertex is listed
   // once per level it is in; four levels of it fit, or all 16 for up to 16 sources (what
   // the caller falls back to).

@@ -27,7 +27,7 @@
 // above hub_deg edges are listed as hub_chunk-edge pieces when their level is formed (the
 // list is kept for the backward sweep), and their partial sums meet in an FP64 scratch.
 //
-// Before and now: R-MAT 20, 256 sources 74.1 -> 24.9 ms; 1000 ER graphs, 16 sources each
+// Before and now: R-MAT 20, 256 sources 74.1 -> 23.3 ms; 1000 ER graphs, 16 sources each
 // 81.2 -> 34.7 ms (as one graph instead of a CTA per graph: with a CTA per graph this form
 // took 67 ms); 20 ER graphs of up to 50 thousand vertices, 40 sources each 57 -> 1.9 ms.
 // What bounds it is the latency of masks and rows (issue 35 % active, L2 75 % hits, 9 GB of

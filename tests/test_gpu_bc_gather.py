@@ -63,3 +63,20 @@ def test_many_graphs_as_one(counts, directed):
             assert _close(out[voff[k]:voff[k + 1]], ref), k
         dg.tune_set("bc.cluster", 1)  # a CTA per graph
         assert _close(dg.bc_graphs(voff, np.array(soff, np.int32), s), out)
+
+
+def test_large_graph_with_wide_pieces():
+    # above the size from which hubs are cut into fewer, longer pieces: dependencies as with
+    # the small pieces (sums of the same terms, so to FP64 rounding before the FP32 store) and
+    # as the oracle's
+    g = G.rmat(19, 14, seed=6)
+    assert g.E > 12_000_000 and np.diff(g.indexofNodes).max() > 2048
+    srcs = G.pick_sources(g, 3, seed=1)
+    with DeviceGraph.from_csr(g, with_weights=False) as dg:
+        wide = dg.bc(srcs).astype(np.float64)
+        dg.tune_set("bc.hub_deg", 64)
+        dg.tune_set("bc.hub_chunk", 64)
+        small = dg.bc(srcs).astype(np.float64)
+    ref = O.bc(g.indexofNodes, g.edgeList, srcs)
+    assert np.all(np.abs(wide - small) <= 2.0**-22 * np.abs(small))
+    assert np.all(np.abs(wide - ref) <= 1e-5 * np.abs(ref) + 1e-6)
