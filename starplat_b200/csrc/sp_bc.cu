@@ -823,7 +823,7 @@ struct GraphsArgs {
   int* cnt;
   double* bc;             // [Vtot] FP64 accumulator (global ids)
   int vmax, cap, maxd;
-  int* err;
+  int* err;               // a word per team: all of a team read the same one and leave together
 };
 
 // The graphs of one team, slot `slot`; k(): the next queue position, the same for all of
@@ -844,7 +844,7 @@ __device__ __forceinline__ void run_graphs(const GraphsArgs& a, int slot, S& syn
     W.lo = a.lo + (size_t)slot * (a.maxd + 2);
     W.maxd = a.maxd;
     W.cnt = a.cnt + slot;
-    W.err = a.err;
+    W.err = a.err + slot;
     W.adj = a.adj;
     W.radj = a.radj;
     W.sym = a.sym;
@@ -1534,7 +1534,7 @@ static int bc_graph_teams(sp_graph* g, int ngraphs, const std::vector<int32_t>& 
   SP_TRY(p->cnt.alloc(ctas + 1));
   SP_TRY(p->bc.alloc(g->V));
   SP_TRY(p->srcs.alloc(std::max(1, nsrc) + 2 * (ngraphs + 1) + ngraphs));
-  SP_TRY(p->err.alloc(1));
+  SP_TRY(p->err.alloc(ctas));
   SP_TRY(p->fout.alloc(g->V));
   int32_t* d_srcs = p->srcs.p;
   int32_t* d_voff = d_srcs + std::max(1, nsrc);
@@ -1547,7 +1547,7 @@ static int bc_graph_teams(sp_graph* g, int ngraphs, const std::vector<int32_t>& 
   bc::k_zero<<<num_sms() * 8, 256, 0, s>>>(p->bc.p, (size_t)g->V);
   g_launches++;
   SP_CHECK_CUDA(cudaMemsetAsync(p->cnt.p, 0, sizeof(int) * (ctas + 1), s));
-  SP_CHECK_CUDA(cudaMemsetAsync(p->err.p, 0, sizeof(int), s));
+  SP_CHECK_CUDA(cudaMemsetAsync(p->err.p, 0, sizeof(int) * ctas, s));
   bc::GraphsArgs a;
   a.off = g->off.p;
   a.adj = g->adj.p;
@@ -1594,8 +1594,9 @@ static int bc_graph_teams(sp_graph* g, int ngraphs, const std::vector<int32_t>& 
 #undef SP_BC_CLUSTERS
   }
   SP_CHECK_LAUNCH();
-  int herr = 0;
-  SP_TRY(copy_out(&herr, p->err.p, sizeof(int), s));
+  std::vector<int> team_err(ctas);
+  SP_TRY(copy_out(team_err.data(), p->err.p, sizeof(int) * ctas, s));
+  const int herr = *std::max_element(team_err.begin(), team_err.end());
   if (herr == 1 && SW > 16) return bc_graph_teams(g, ngraphs, voff, soff, hs, vmax, smax, 16, BC);
   if (herr) {
     set_error("sp_bc_graphs: device error %d (1 level lists full, 2 deeper than %d levels)", herr, maxd);

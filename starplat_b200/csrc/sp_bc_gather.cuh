@@ -69,7 +69,7 @@ struct Gather {
   int maxd;
   int* cnt;             // entries appended
   double* bc;           // [V]
-  int* err;             // 1 a list is full, 2 too deep, 3 barrier timeout
+  int* err;             // this team's own: 1 a list is full, 2 too deep, 3 barrier timeout
   // entries with more than hub_deg edges, as pieces {vertex, entry, first edge, end}; pcap = 0:
   // none split.
   // [0] by out-edges, kept for all levels (plo / hlo: level starts); [1] by in-edges, for
@@ -561,8 +561,10 @@ __device__ bool gather_batch(const Gather& G, const int32_t* srcs, const int32_t
     G.mask[v] = z;
     G.back[v] = G.back[G.bstride + v] = 0ull;
   }
-  // a full list (err 1) truncated this batch: every team member reads the flag after the
-  // last barrier (nothing writes it after that), so all leave together
+  // a full list (err 1) truncated this batch: the whole team reads its flag after its last
+  // barrier. No other team has the same word, so nothing writes it after that barrier and
+  // all leave together: a CTA that stayed would wait for, or read the shared memory of, one
+  // that has left.
   if (!sync.sync()) return false;
   return ld_now(G.err) == 0;
 }
