@@ -1024,6 +1024,14 @@ __global__ void k_collect_marked(int V, const uint8_t* __restrict__ bad, const i
     if (bad[v] && dist[v] != INT_MAX) seeds[atomicAdd(nseeds, 1)] = v;
 }
 
+// Sources of added edges that are not marked: a marked one is a seed already, or has no
+// distance to add to. Queues hold V entries, so no vertex may be a seed twice.
+__global__ void k_collect_adds(int n, const int32_t* __restrict__ src, const uint8_t* __restrict__ bad,
+                               int32_t* seeds, int* nseeds) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    if (!bad[src[i]]) seeds[atomicAdd(nseeds, 1)] = src[i];
+}
+
 __global__ void k_count_marked(int V, const uint8_t* __restrict__ bad, int* count) {
   int c = 0;
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) c += bad[v];
@@ -1597,8 +1605,10 @@ extern "C" int sp_sssp_dynamic(sp_graph_h g, int64_t n, const char* type, const 
     SP_CHECK_CUDA(cudaMemcpyAsync(p->dist.p, old_dist.p, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, s));
     std::vector<int32_t> add_src(seeds);
     int nseed = 0;
-    dbuf<int32_t> d_seeds, anc;
-    SP_TRY(d_seeds.alloc((size_t)V + add_src.size() + 1));
+    std::sort(add_src.begin(), add_src.end());
+    add_src.erase(std::unique(add_src.begin(), add_src.end()), add_src.end());
+    dbuf<int32_t> d_seeds, d_adds, anc;
+    SP_TRY(d_seeds.alloc((size_t)V));
     if (nb > 0) {
       int passes = 1;
       while (passes < 32 && (1ll << (passes - 1)) < (long long)V) ++passes;
@@ -1627,14 +1637,20 @@ extern "C" int sp_sssp_dynamic(sp_graph_h g, int64_t n, const char* type, const 
       ss::k_collect_marked<<<num_sms() * 8, 256, 0, s>>>(V, marked, p->dist.p, d_seeds.p, nbad.p + 1);
       SP_CHECK_LAUNCH();
       g_launches += 3;
+      if (!add_src.empty()) {
+        SP_TRY(d_adds.alloc(add_src.size()));
+        SP_CHECK_CUDA(cudaMemcpyAsync(d_adds.p, add_src.data(), sizeof(int32_t) * add_src.size(),
+                                      cudaMemcpyHostToDevice, s));
+        ss::k_collect_adds<<<num_sms() * 2, 256, 0, s>>>((int)add_src.size(), d_adds.p, marked, d_seeds.p,
+                                                         nbad.p + 1);
+        SP_CHECK_LAUNCH();
+      }
       SP_TRY(copy_out(&nseed, nbad.p + 1, sizeof(int), s));
-    }
-    std::sort(add_src.begin(), add_src.end());
-    add_src.erase(std::unique(add_src.begin(), add_src.end()), add_src.end());
-    if (!add_src.empty())
-      SP_CHECK_CUDA(cudaMemcpyAsync(d_seeds.p + nseed, add_src.data(), sizeof(int32_t) * add_src.size(),
+    } else if (!add_src.empty()) {
+      SP_CHECK_CUDA(cudaMemcpyAsync(d_seeds.p, add_src.data(), sizeof(int32_t) * add_src.size(),
                                     cudaMemcpyHostToDevice, s));
-    nseed += (int)add_src.size();
+      nseed = (int)add_src.size();
+    }
     g->sssp_last_incremental = 2;
     if (nseed == 0) return copy_out(dist, p->dist.p, sizeof(int32_t) * V, s);
     return sssp_delta(g, w, source, dist, delta, ctas, local, nullptr, d_seeds.p, nseed);
