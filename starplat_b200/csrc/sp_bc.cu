@@ -1015,6 +1015,18 @@ struct BcPlan {
   int64_t vmax = 0, vsq = 0, vrows[4] = {}, vedges[4] = {};
   int var_choice = -1, var_nsrc = 0;
   unsigned var_gen = 0;
+  // Gives back the gather form's rows, masks and lists.
+  void release_state() {
+    sigma.release();
+    dacc.release();
+    masks.release();
+    flv.release();
+    flm.release();
+    piece.release();
+    rpiece.release();
+    hub.release();
+    rhub.release();
+  }
 };
 
 int bc_hub_deg_default() { return bc::HUB_DEG; }
@@ -1679,12 +1691,13 @@ extern "C" int sp_bc_graphs(sp_graph_h g, int32_t ngraphs, const int32_t* vertex
                      (int)boff.size() - 1);
       if (st != SP_ERR_UNSUPPORTED || width <= 16) break;  // full lists: 16 sources a graph always fit
     }
-    if (st != SP_ERR_OOM) {  // without the memory: teams
+    if (st != SP_ERR_OOM) {
       SP_TRY(st);
       bc::k_to_float<<<num_sms() * 4, 256, 0, s>>>(p->bc.p, p->fout.p, g->V);
       SP_CHECK_LAUNCH();
       return copy_out(BC, p->fout.p, sizeof(float) * g->V, s);
     }
+    p->release_state();  // without the memory: teams, whose state is smaller
   }
   const int SW = smax > 32 ? 64 : smax > 16 ? 32 : 16;
   return bc_graph_teams(g, ngraphs, voff, soff, hs, vmax, smax, SW, BC);

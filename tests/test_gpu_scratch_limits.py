@@ -1,0 +1,54 @@
+"""GPU: calls whose fastest form does not fit the free device memory run in a form that does.
+Each test leaves a given number of bytes free (the rest is held by one allocation) and
+compares with the same call made with all memory."""
+import contextlib
+
+import numpy as np
+import pytest
+
+from starplat_b200 import _lib
+from starplat_b200 import generators as G
+from starplat_b200.device import DeviceGraph
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+
+
+@contextlib.contextmanager
+def _only(free_bytes):
+    """All but free_bytes of the device's free memory held for the block's time."""
+    import torch
+
+    _lib.lib().sp_cache_trim(None)
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - free_bytes, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del held
+        torch.cuda.empty_cache()
+
+
+def test_many_graphs_when_their_union_does_not_fit():
+    # 300 random graphs of 8,000 vertices, 40 sources each: the union's rows, scratch, masks
+    # and lists take 3.0 GB, a team per graph 1.8 GB; what the union had taken before it
+    # failed must not be in the teams' way
+    n, ng, k = 8000, 300, 40
+    rng = np.random.default_rng(3)
+    m = 2 * n
+    u = rng.integers(0, n, (ng, m), dtype=np.int64) + n * np.arange(ng)[:, None]
+    v = rng.integers(0, n, (ng, m), dtype=np.int64) + n * np.arange(ng)[:, None]
+    u, v = u.ravel()[(u != v).ravel()], v.ravel()[(u != v).ravel()]
+    V = n * ng
+    key = np.unique(np.concatenate([u * V + v, v * V + u]))
+    off = np.searchsorted(key, np.arange(V + 1) * V).astype(np.int32)
+    adj = (key % V).astype(np.int32)
+    voff = (n * np.arange(ng + 1)).astype(np.int32)
+    soff = (k * np.arange(ng + 1)).astype(np.int32)
+    srcs = np.concatenate([np.sort(rng.choice(n, k, replace=False)) + b for b in voff[:-1]]).astype(np.int32)
+    with DeviceGraph(off, adj, None, off, adj) as dg:
+        ref = dg.bc_graphs(voff, soff, srcs).astype(np.float64)
+    with DeviceGraph(off, adj, None, off, adj) as dg:
+        with _only(2850 * MB):
+            out = dg.bc_graphs(voff, soff, srcs).astype(np.float64)
+    assert np.all(np.abs(out - ref) <= 1e-5 * np.abs(ref) + 1e-6)
