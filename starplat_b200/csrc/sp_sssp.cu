@@ -1285,18 +1285,24 @@ static int sssp_delta_batches(sp_graph* g, const int32_t* w, const std::vector<i
     const size_t per_src = (size_t)9 * 4 * (size_t)V + (size_t)V / 2 + 4096;
     B = (int)std::max<size_t>(1, std::min<size_t>(B, (total_b / 8) / per_src));
   }
-  const int gsz = total / B;
-  const size_t BV = (size_t)B * V;
   Arena A;
   const int nwords = (V + 31) / 32;
   dspan<int32_t> dist, q0, q1, f0, f1, h0, h1, hb0, hb1, dsrc;
   dspan<unsigned> bits;
   dspan<ss::Ctl> ctl;
-  for (dspan<int32_t>* d : {&dist, &q0, &q1, &f0, &f1, &h0, &h1, &hb0, &hb1}) A.want(*d, BV);
-  A.want(bits, (size_t)4 * nwords * B);
-  A.want(dsrc, B);
-  A.want(ctl, B);
-  SP_TRY(A.commit());
+  for (;; B /= 2) {  // fewer sources at a time where the memory that is free holds no more
+    const size_t BV = (size_t)B * V;
+    A.reqs.clear();
+    A.size = 0;
+    for (dspan<int32_t>* d : {&dist, &q0, &q1, &f0, &f1, &h0, &h1, &hb0, &hb1}) A.want(*d, BV);
+    A.want(bits, (size_t)4 * nwords * B);
+    A.want(dsrc, B);
+    A.want(ctl, B);
+    const int st = A.commit();
+    if (st == SP_OK) break;
+    if (st != SP_ERR_OOM || B == 1) return st;
+  }
+  const int gsz = total / B;
   ss::Args a;
   a.off = g->off.p;
   a.adj = g->adj.p;

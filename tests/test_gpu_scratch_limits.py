@@ -52,3 +52,17 @@ def test_many_graphs_when_their_union_does_not_fit():
         with _only(2850 * MB):
             out = dg.bc_graphs(voff, soff, srcs).astype(np.float64)
     assert np.all(np.abs(out - ref) <= 1e-5 * np.abs(ref) + 1e-6)
+
+
+def test_batched_sssp_with_less_memory_than_a_full_batch():
+    # a batch of 8 sources takes 8 * 37 bytes a vertex (1.2 GB here), 4 half of that
+    g = G.grid(2048, 2048)
+    g.edgeLen = G.hash_weights(g, 3, 1, 50, True)
+    srcs = np.array([5, 77777, 2049, 4000000, 12345, 2000000, 3, 1048576], np.int32)
+    with DeviceGraph.from_csr(g) as dg:
+        dg.sssp(0)  # what a single solve keeps
+        with _only(900 * MB):
+            out = dg.sssp_batch(srcs)
+        assert dg.tune_get("sssp.last_batch") == 4
+        assert np.array_equal(out, dg.sssp_batch(srcs))
+        assert dg.tune_get("sssp.last_batch") == 8
