@@ -1021,8 +1021,9 @@ static int tc_count_part(sp_graph* g, int part, int nparts, int64_t* triangle_co
   g->last_variant[VAR_TC] = cand;
   const bool dflt = g->V <= 65536 ? g->E > RANK_MIN_E && cta_warps == tc::CTA_WARPS_DEFAULT : wu == tc::WU_DEFAULT;
   if (g->symmetric == 1 && dflt) {
-    SP_TRY(build_rank_plan(g));
-    return rank_count(g, part, nparts, triangle_count, nullptr);
+    const int st = build_rank_plan(g);
+    if (st == SP_OK) return rank_count(g, part, nparts, triangle_count, nullptr);
+    if (st != SP_ERR_OOM) return st;  // making it takes 26 bytes an entry, the oriented lists' plan 10
   }
   SP_TRY(build_tc_plan(g));
   if (nparts == 1) return tc_count(g, g->tc->order.p, g->V, cta_warps, wu, triangle_count);
@@ -1036,8 +1037,9 @@ static int tc_count_part(sp_graph* g, int part, int nparts, int64_t* triangle_co
 static int lcc_count_part(sp_graph* g, int part, int nparts, int* counts) {
   SP_TRY(ensure_symmetry(g));
   if (g->symmetric == 1) {
-    SP_TRY(build_rank_plan(g));
-    return rank_count(g, part, nparts, nullptr, counts);
+    const int st = build_rank_plan(g);
+    if (st == SP_OK) return rank_count(g, part, nparts, nullptr, counts);
+    if (st != SP_ERR_OOM) return st;
   }
   SP_TRY(build_tc_plan(g));
   if (g->V) SP_CHECK_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * g->V, g->stream));

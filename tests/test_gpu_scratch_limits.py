@@ -66,3 +66,17 @@ def test_batched_sssp_with_less_memory_than_a_full_batch():
         assert dg.tune_get("sssp.last_batch") == 4
         assert np.array_equal(out, dg.sssp_batch(srcs))
         assert dg.tune_get("sssp.last_batch") == 8
+
+
+def test_triangles_when_the_rank_plan_does_not_fit():
+    # making the lists in rank order takes about 26 bytes an entry (800 MB), the oriented
+    # lists of the other kernels 10
+    g = G.rmat(20, 16, seed=4)
+    with DeviceGraph.from_csr(g, with_weights=False) as dg:
+        count, per = dg.tc(), dg.clustering_coeff()
+    for call, ref in (("tc", count), ("clustering_coeff", per)):
+        with DeviceGraph.from_csr(g, with_weights=False) as dg:
+            dg.info()  # the symmetry
+            with _only(550 * MB):
+                assert np.array_equal(getattr(dg, call)(), ref), call
+            assert np.array_equal(getattr(dg, call)(), ref), call
