@@ -121,8 +121,8 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "sssp.delta"  SSSP bucket width used when sp_sssp gets delta <= 0 (0 = the largest
  *             edge weight).
  *   "sssp.ctas_per_sm"  SSSP: persistent CTAs per SM of the delta-stepping kernel (1..8,
- *             default 4; at most the 3 that are resident run; fewer make each grid barrier
- *             cheaper on high-diameter graphs).
+ *             default 4; at most the 3 that are resident run, so 3 to 8 and "sssp.last_ctas"
+ *             4 are the same; fewer make each grid barrier cheaper on high-diameter graphs).
  *   "sssp.batch"  sp_sssp_batch / sp_closeness: sources per cooperative launch, each on
  *             its own group of CTAs (1..1024, default 8; capped by the co-resident CTAs
  *             and by 1/8 of device memory at 44 bytes per vertex per source).
@@ -131,9 +131,10 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *             last SSSP call ran; "sssp.last_relaxed": the edges it relaxed (each
  *             out-edge of a vertex once per time the vertex was expanded).
  *   "tc.cta_warps"  TC on graphs of up to 65536 vertices: 0 = a bitmap per warp;
- *             2, 4, 8 or 16 = one bitmap per CTA of that many warps sharing each anchor.
- *             At the default (4) symmetric graphs are counted in rank order instead (the
- *             count itself from 65536 vertices or 131072 entries on).
+ *             2, 4, 8 or 16 = one bitmap per CTA of that many warps sharing each anchor; -1
+ *             (default) = rank order on symmetric graphs of more than 131072 entries, else 4.
+ *   "tc.unroll"  TC on larger graphs: 1, 2 or 4 = the hash kernel with that many probe-list
+ *             elements per lane in flight; -1 (default) = rank order on symmetric graphs, else 4.
  *   "tc.last_incremental" (read only): 1 if the last sp_tc_dynamic counted only the
  *             triangles through the batch's edges, 0 if it counted the graph again.
  *   "sssp.hub_deg", "sssp.hub_chunk"  SSSP: queued vertices with more out-edges than
@@ -173,7 +174,7 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "bc.pull_alpha"  factor of the bc.dir = 1 rule, in thousandths (default 1000).
  *   "bc.trace"  1: record per level (entries, their out-edges, unreached in-edges, pull)
  *             and the device timer; read with sp_bc_level_trace.
- *   "bc.cluster"  BC of many graphs (sp_bc_graphs): unset, all graphs run as one; set, CTAs
+ *   "bc.cluster"  BC of many graphs (sp_bc_graphs): 0 (default), all graphs run as one; CTAs
  *             per graph, 1, 2, 4 or 8; above 1 the CTAs of a thread-block cluster share a graph
  *             and synchronise with hardware cluster barriers. */
 int sp_tune_set(sp_graph_h g, const char* key, int64_t value);

@@ -1,7 +1,8 @@
 """Autotuner for the schedule knobs (sp_tune_set) of one graph.
 
 Each algorithm's kernels take thresholds that change only how work is split:
-  tc        tc.cta_warps: a bitmap per warp (0) or per CTA of 2 / 4 / 8 warps
+  tc        tc.cta_warps: the library's choice (-1: rank order on larger symmetric graphs), a
+            bitmap per warp (0) or per CTA of 2 / 4 / 8 warps
   pagerank  pr.order: vertex order by out-degree (0) or in-degree class first (1);
             pr.src_hint: L1 policy of the srcList loads; pr.hot: sources of the
             L1-resident hot phase (0 = one phase); pr.l1_hot: sources whose gathers
@@ -26,7 +27,7 @@ from typing import Callable, Dict, List, Sequence, Tuple
 import numpy as np
 
 KNOBS: Dict[str, Dict[str, Sequence[int]]] = {
-    "tc": {"tc.cta_warps": (0, 2, 4, 8)},
+    "tc": {"tc.cta_warps": (-1, 0, 2, 4, 8)},
     "pagerank": {"pr.order": (0, 1), "pr.src_hint": (0, 2), "pr.hot": (0, 4096), "pr.l1_hot": (0, 32768, 131072)},
     "sssp": {"sssp.hub_deg": (64, 128, 512, 2048), "sssp.hub_chunk": (32, 64, 256), "sssp.local": (0, 16, 64)},
     "bc": {"bc.hub_deg": (32, 64, 256, 4096), "bc.hub_chunk": (64, 128, 256), "bc.dir": (0, 1)},

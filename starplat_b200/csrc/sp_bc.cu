@@ -1029,10 +1029,6 @@ struct BcPlan {
   }
 };
 
-int bc_hub_deg_default() { return bc::HUB_DEG; }
-int bc_cluster_default() { return bc::CLUSTER_DEFAULT; }
-int bc_hub_chunk_default() { return bc::HUB_CHUNK; }
-
 void free_bc_plan(BcPlan* p) { delete p; }
 
 // ---- learned kernel variant -------------------------------------------------------
@@ -1121,12 +1117,25 @@ static int bc_variant_pick(sp_graph* g, int nsrc, int* cand) {
   return SP_OK;
 }
 
-// bc.hub_deg / bc.hub_chunk of a call: the knobs, the learned variant, or the defaults
-// (wide: those of the gathering form on large graphs, where neither knob is set).
-static int bc_split(sp_graph* g, int nsrc, int* hub_deg, int* hub_chunk, bool wide = false) {
-  wide = wide && g->bc_hub_deg <= 0 && g->bc_hub_chunk <= 0;
+// The forward direction policy of a call: the knob, or the level model where one is loaded;
+// 0 is the gather form.
+static int bc_direction(sp_graph* g) {
+  std::vector<float> packed;
+  return g->bc_dir >= 0 ? g->bc_dir : mlp_level_model(packed) ? 4 : bc::DIR_DEFAULT;
+}
+
+// bc.hub_deg / bc.hub_chunk of g: the knobs, or the defaults (others for the gather form on
+// large graphs, where neither knob is set).
+void bc_hub_split(sp_graph* g, int* hub_deg, int* hub_chunk) {
+  const bool wide =
+      (double)g->E >= bc::WIDE_E && g->bc_hub_deg <= 0 && g->bc_hub_chunk <= 0 && bc_direction(g) == 0;
   *hub_deg = g->bc_hub_deg > 0 ? g->bc_hub_deg : wide ? bc::WIDE_HUB_DEG : bc::HUB_DEG;
   *hub_chunk = g->bc_hub_chunk > 0 ? g->bc_hub_chunk : wide ? bc::WIDE_HUB_CHUNK : bc::HUB_CHUNK;
+}
+
+// The same for a call, with the learned variant.
+static int bc_split(sp_graph* g, int nsrc, int* hub_deg, int* hub_chunk) {
+  bc_hub_split(g, hub_deg, hub_chunk);
   int cand = -1;
   SP_TRY(bc_variant_pick(g, nsrc, &cand));
   if (cand >= 0) {
@@ -1159,7 +1168,7 @@ static int bc_gather(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch, in
   const size_t cap = (size_t)V * std::min(width, 16) + 1024;  // level-list entries (vertex, mask)
   bc::GatherArgs a;
   bc::Gather& W = a.G;
-  SP_TRY(bc_split(g, nsrc, &W.hub_deg, &W.hub_chunk, (double)g->E >= bc::WIDE_E));
+  SP_TRY(bc_split(g, nsrc, &W.hub_deg, &W.hub_chunk));
   // Pieces of one pass over the graph: at most E / chunk + E / hub_deg. A vertex is listed
   // once per level it is in; four levels of it fit, or all 16 for up to 16 sources (what
   // the caller falls back to).
@@ -1255,14 +1264,9 @@ static int bc_gather(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch, in
 // the level model; bc.dir = 0 (the default without a model) takes the gather form.
 static int bc_grid(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch_hint, int32_t* lvl_out = nullptr,
                    double* sig_out = nullptr) {
-  {
-    std::vector<float> packed;
-    const unsigned lgen = mlp_level_model(packed);
-    if ((g->bc_dir >= 0 ? g->bc_dir : (lgen ? 4 : bc::DIR_DEFAULT)) == 0)
-    {
-      const int batch = std::max(1, std::min(std::min(batch_hint, 64), nsrc));
-      return bc_gather(g, d_srcs, nsrc, batch, batch, 1 << 14, lvl_out, sig_out);
-    }
+  if (bc_direction(g) == 0) {
+    const int batch = std::max(1, std::min(std::min(batch_hint, 64), nsrc));
+    return bc_gather(g, d_srcs, nsrc, batch, batch, 1 << 14, lvl_out, sig_out);
   }
   BcPlan* p = g->bc;
   cudaStream_t s = g->stream;

@@ -778,8 +778,8 @@ int sp_tune_set(sp_graph_h g, const char* key, int64_t value) {
     return SP_OK;
   }
   if (!strcmp(key, "tc.cta_warps")) {
-    if (value != 0 && value != 2 && value != 4 && value != 8 && value != 16) {
-      set_error("sp_tune_set: tc.cta_warps must be 0, 2, 4, 8 or 16");
+    if (value != -1 && value != 0 && value != 2 && value != 4 && value != 8 && value != 16) {
+      set_error("sp_tune_set: tc.cta_warps must be -1, 0, 2, 4, 8 or 16");
       return SP_ERR_INVALID;
     }
     g->tc_cta_warps = (int32_t)value;
@@ -794,8 +794,8 @@ int sp_tune_set(sp_graph_h g, const char* key, int64_t value) {
     return SP_OK;
   }
   if (!strcmp(key, "tc.unroll")) {
-    if (value != 1 && value != 2 && value != 4) {
-      set_error("sp_tune_set: tc.unroll must be 1, 2 or 4");
+    if (value != -1 && value != 1 && value != 2 && value != 4) {
+      set_error("sp_tune_set: tc.unroll must be -1, 1, 2 or 4");
       return SP_ERR_INVALID;
     }
     g->tc_unroll = (int32_t)value;
@@ -945,19 +945,23 @@ int sp_tune_get(sp_graph_h g, const char* key, int64_t* value) {
     return SP_OK;
   }
   if (!strcmp(key, "bc.cluster")) {
-    *value = g->bc_cluster > 0 ? g->bc_cluster : bc_cluster_default();
+    *value = g->bc_cluster;
     return SP_OK;
   }
   if (!strcmp(key, "bc.hub_deg")) {
-    *value = g->bc_hub_deg > 0 ? g->bc_hub_deg : bc_hub_deg_default();
+    int deg, chunk;
+    bc_hub_split(g, &deg, &chunk);
+    *value = deg;
     return SP_OK;
   }
   if (!strcmp(key, "bc.hub_chunk")) {
-    *value = g->bc_hub_chunk > 0 ? g->bc_hub_chunk : bc_hub_chunk_default();
+    int deg, chunk;
+    bc_hub_split(g, &deg, &chunk);
+    *value = chunk;
     return SP_OK;
   }
   if (!strcmp(key, "tc.cta_warps")) {
-    *value = g->tc_cta_warps >= 0 ? g->tc_cta_warps : tc_cta_warps_default();
+    *value = g->tc_cta_warps;
     return SP_OK;
   }
   if (!strcmp(key, "bc.batch")) {
@@ -965,7 +969,7 @@ int sp_tune_get(sp_graph_h g, const char* key, int64_t* value) {
     return SP_OK;
   }
   if (!strcmp(key, "tc.unroll")) {
-    *value = g->tc_unroll > 0 ? g->tc_unroll : 4;
+    *value = g->tc_unroll;
     return SP_OK;
   }
   if (!strcmp(key, "lv.cta_slots")) {

@@ -188,16 +188,16 @@ struct sp_graph {
   int32_t sssp_last_epochs = 0;  // bucket advances of the last single-source solve
   int32_t sssp_last_epolicy = 0;  // the width policy the last solve ran
   int32_t sssp_last_batch = 0;  // sources per launch of the last batched run (reporting)
-  int32_t tc_cta_warps = -1;  // TC: warps per CTA of the shared-bitmap kernel (-1 = default, 0 = off)
+  int32_t tc_cta_warps = -1;  // TC: warps per CTA of the shared-bitmap kernel (-1 = the library's choice, 0 = off)
   int32_t bc_dir = -1;        // BC forward direction policy (-1 = default)
   int32_t bc_pull_alpha = 0;  // BC pull rule factor in thousandths (0 = default)
   int32_t bc_dir_seed = 0;    // BC direction exploration seed
   int32_t bc_trace = 0;       // 1: record the per-level trace of the grid form
-  int32_t bc_batch = 0;
+  int32_t bc_batch = 0;      // BC: sources per multi-source batch (0 = 64)
   int32_t bc_hub_deg = 0;  // BC: split level-list entries above this degree (0 = default)
   int32_t bc_hub_chunk = 0;  // BC: edges per piece of a split entry (0 = default)
-  int32_t bc_cluster = 0;    // BC many-graphs form: CTAs per graph (0 = default)    // BC sources per multi-source batch (0 = 64)
-  int32_t tc_unroll = -1;    // TC hash path: probe-list elements per lane per pass (-1 = default)
+  int32_t bc_cluster = 0;    // BC of many graphs: CTAs per graph (0 = all graphs as one)
+  int32_t tc_unroll = -1;    // TC hash path: probe-list elements per lane per pass (-1 = the library's choice)
   int32_t lv_cta_slots = -1;  // Louvain: shared table slots of the CTA bin (-1 = default)
   int32_t lv_trace = 0;       // 1: record the per-level trace of sp_louvain
   // learned kernel variants, per algorithm (pr, tc, bc, lv): -1 learned when a variant
@@ -230,14 +230,12 @@ int pr_order_default();               // PageRank vertex order default (sp_pager
 int pr_src_hint_default();
 int pr_l1_hot_default();
 int pr_vec_default();
-int tc_cta_warps_default();           // TC kernel choice default (sp_tc.cu)
-int bc_hub_deg_default();             // BC entry-splitting defaults (sp_bc.cu)
+// BC: hub_deg and hub_chunk that the knobs or the defaults give on g (sp_bc.cu)
+void bc_hub_split(sp_graph* g, int* hub_deg, int* hub_chunk);
 int sssp_hub_deg_default();           // SSSP hub-splitting defaults (sp_sssp.cu)
 int sssp_hub_chunk_default();
 int sssp_local_default();
 int sssp_batch_default();         // batched SSSP sources per launch (sp_sssp.cu)
-int bc_hub_chunk_default();
-int bc_cluster_default();
 int ensure_symmetry(sp_graph* g);     // fills g->symmetric
 int copy_out(void* dst, const void* src, size_t bytes, cudaStream_t s);  // host or device dst
 // SSSP helpers shared with the split solve (sp_sssp.cu): the weights on the device (the

@@ -702,8 +702,6 @@ struct TcPlan {
   unsigned var_gen = 0;
 };
 
-int tc_cta_warps_default() { return tc::CTA_WARPS_DEFAULT; }
-
 void free_tc_plan(TcPlan* p) {
   if (!p) return;
   p->ooff.release();
@@ -1004,9 +1002,10 @@ static int order_part(sp_graph* g, int part, int nparts, dbuf<int32_t>& out, int
 constexpr int64_t RANK_MIN_E = 1 << 17;
 
 // The triangles of part `part` of `nparts`. Symmetric graphs count in rank order
-// (sp_tc_rank.cuh, with the times of both) unless a knob or variant asks for a kernel
-// other than the default. The bitmap and hash kernels run the directed graphs, whose
-// anchors and probes the formula fixes.
+// (sp_tc_rank.cuh, with the times of both) unless a variant is forced or learned, or the knob
+// of the bitmap (up to 65536 vertices) or hash kernel is set: each of those runs the kernel
+// it names. The bitmap and hash kernels run the directed graphs, whose anchors and probes
+// the formula fixes.
 static int tc_count_part(sp_graph* g, int part, int nparts, int64_t* triangle_count) {
   SP_TRY(ensure_symmetry(g));
   if (!g->tc) g->tc = new TcPlan();
@@ -1019,7 +1018,7 @@ static int tc_count_part(sp_graph* g, int part, int nparts, int64_t* triangle_co
     else wu = tc::VARIANTS[cand].wu;
   }
   g->last_variant[VAR_TC] = cand;
-  const bool dflt = g->V <= 65536 ? g->E > RANK_MIN_E && cta_warps == tc::CTA_WARPS_DEFAULT : wu == tc::WU_DEFAULT;
+  const bool dflt = cand < 0 && (g->V <= 65536 ? g->E > RANK_MIN_E && g->tc_cta_warps < 0 : g->tc_unroll <= 0);
   if (g->symmetric == 1 && dflt) {
     const int st = build_rank_plan(g);
     if (st == SP_OK) return rank_count(g, part, nparts, triangle_count, nullptr);
