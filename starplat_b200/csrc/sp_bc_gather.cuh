@@ -452,10 +452,12 @@ __device__ bool gather_batch(const Gather& G, const int32_t* srcs, const int32_t
     if (!sync.sync()) return false;
   }
   // ---- forward
-  int d = 0, p0 = 0, h0 = 0;
-  while (true) {
-    const int b = ld_now(G.lo + d), e = ld_now(G.lo + d + 1);
-    if (b == e) break;
+  // A level's counters are read once per CTA: while every warp of the grid read them (six
+  // loads of one sector by 4,700 warps), they took a quarter of a deep graph's time (levels of
+  // a 300 x 300 grid from one source 7.4 ms, 5.6 without).
+  __shared__ int s_now[5];
+  int d = 0, p0 = 0, h0 = 0, b = 0, e = nsrc;
+  while (b != e) {
     if (d + 2 > G.maxd) {
       if (gt == 0) atomicExch(G.err, 2);
       return false;
@@ -463,10 +465,13 @@ __device__ bool gather_batch(const Gather& G, const int32_t* srcs, const int32_t
     int p1 = 0, h1 = 0, rp1 = 0, rh1 = 0;
     const int half = d & 1;
     if (G.pcap) {
-      p1 = min(ld_now(G.pc), G.pcap);
-      h1 = min(ld_now(G.pc + 1), G.hcap);
-      rp1 = min(ld_now(G.pc + 2 + half), G.pcap);
-      rh1 = min(ld_now(G.pc + 4 + half), G.hcap);
+      const int k = threadIdx.x;
+      if (k < 4) s_now[k] = ld_now(G.pc + (k < 2 ? k : 2 * k - 2 + half));
+      __syncthreads();
+      p1 = min(s_now[0], G.pcap);
+      h1 = min(s_now[1], G.hcap);
+      rp1 = min(s_now[2], G.pcap);
+      rh1 = min(s_now[3], G.hcap);
       if (gt == 0) {
         G.plo[d + 1] = p1;
         G.hlo[d + 1] = h1;
@@ -479,18 +484,18 @@ __device__ bool gather_batch(const Gather& G, const int32_t* srcs, const int32_t
                           gw, nw, pk);
     if (!sync.sync()) return false;
     // the next level's masks and pieces, and the path counts of this level's split entries
-    const int c = min(ld_now(G.cnt), G.cap);
+    if (threadIdx.x == 0) s_now[4] = ld_now(G.cnt);
+    __syncthreads();
+    const int c = min(s_now[4], G.cap);
     if (gt == 0) G.lo[d + 2] = c;
     if (G.pcap && !G.sym && gt == 0) G.pc[2 + half] = G.pc[4 + half] = 0;  // read by all before the barrier
     for (int i0 = e + gw * 32; i0 < c; i0 += nw * 32) {
       const int k = i0 + lane;
-      int w = 0;
+      const int w = k < c ? G.flv[k] : 0;
       if (k < c) {
-        w = G.flv[k];
-        const unsigned long long mk = G.mask[w].nxt;
-        G.flm[k] = mk;
-        G.mask[w].seen |= mk;
-        G.mask[w].nxt = 0ull;
+        const Masks x = ld_masks(G.mask + w);
+        G.flm[k] = x.nxt;
+        *reinterpret_cast<ulonglong2*>(G.mask + w) = make_ulonglong2(x.seen | x.nxt, 0ull);  // seen, nxt
       }
       if (G.pcap) {
         const int ob = G.off[w], od = G.off[w + 1] - ob;
@@ -516,6 +521,8 @@ __device__ bool gather_batch(const Gather& G, const int32_t* srcs, const int32_t
     if (!sync.sync()) return false;
     p0 = p1;
     h0 = h1;
+    b = e;
+    e = c;
     ++d;
   }
   const int D = d;  // levels 0 .. D - 1

@@ -1,0 +1,50 @@
+"""GPU: BC, levels and path counts on the graphs whose launch or pieces differ by their largest
+degree: rows on both sides of the piece size (64), and grids and rings on both sides of the
+degree (8) up to which fewer CTAs run. Against the oracle: 1e-5 relative, counts exact."""
+import numpy as np
+import pytest
+
+from graphs import from_pairs, star
+from oracle import oracle as O
+from starplat_b200 import generators as G
+from starplat_b200.device import DeviceGraph
+
+pytestmark = pytest.mark.gpu
+
+
+def _ring(n, reach):  # every vertex joined to the next `reach`: degree 2 * reach
+    i = np.repeat(np.arange(n, dtype=np.int32), reach)
+    return from_pairs(n, np.stack([i, (i + np.tile(np.arange(1, reach + 1), n)) % n], 1), symmetrize=True)
+
+
+def _ring9(n):  # degree 8, one vertex of degree 9
+    i = np.repeat(np.arange(n, dtype=np.int32), 4)
+    p = np.stack([i, (i + np.tile(np.arange(1, 5), n)) % n], 1)
+    return from_pairs(n, np.concatenate([p, [[0, n // 2]]]), symmetrize=True)
+
+
+GRAPHS = {
+    "star64": lambda: star(64, directed_in=False),
+    "star65": lambda: star(65, directed_in=False),
+    "ring8": lambda: _ring(3001, 4),
+    "ring9": lambda: _ring9(3001),
+    "ring10": lambda: _ring(2000, 5),
+    "grid": lambda: G.grid(61, 67),
+}
+
+
+@pytest.mark.parametrize("nsrc", [1, 16, 40, 64])
+@pytest.mark.parametrize("name", list(GRAPHS))
+def test_degree_borders(name, nsrc):
+    g = GRAPHS[name]()
+    srcs = G.pick_sources(g, min(nsrc, g.V), seed=4, min_out_degree=0)
+    with DeviceGraph.from_csr(g, with_weights=False) as dg:
+        ref = O.bc(g.indexofNodes, g.edgeList, srcs)
+        for _ in range(2):
+            out = dg.bc(srcs).astype(np.float64)
+            assert np.all(np.abs(out - ref) <= 1e-5 * np.abs(ref) + 1e-9 * max(1.0, ref.max()))
+        lv, sg = dg.bfs_sigma(srcs)
+        for k in (0, len(lv) - 1):
+            rl, rs, _ = O.bfs_sigma(g.indexofNodes, g.edgeList, int(srcs[k]))
+            assert np.array_equal(lv[k], rl)
+            assert np.all(np.abs(sg[k] - rs) <= 1e-12 * rs)  # beyond 2^53 in the deep ones
