@@ -174,8 +174,8 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "bc.pull_alpha"  factor of the bc.dir = 1 rule, in thousandths (default 1000).
  *   "bc.trace"  1: record per level (entries, their out-edges, unreached in-edges, pull)
  *             and the device timer; read with sp_bc_level_trace.
- *   "bc.cluster"  BC of many graphs (sp_bc_graphs): 0 (default), all graphs run as one; CTAs
- *             per graph, 1, 2, 4 or 8; above 1 the CTAs of a thread-block cluster share a graph
+ *   "bc.cluster"  BC of many graphs (sp_bc_graphs): 0 (default), all graphs run as one (small
+ *             grids and roads: a CTA per graph); CTAs per graph, 1, 2, 4 or 8; above 1 the CTAs of a thread-block cluster share a graph
  *             and synchronise with hardware cluster barriers. */
 int sp_tune_set(sp_graph_h g, const char* key, int64_t value);
 int sp_tune_get(sp_graph_h g, const char* key, int64_t* value);

@@ -1637,6 +1637,30 @@ static int bc_graph_teams(sp_graph* g, int ngraphs, const std::vector<int32_t>& 
 }
 }  // namespace sp
 
+namespace sp {
+// Whether graphs without a row above NARROW_DEG (grids, roads) run faster as teams than as one
+// graph: their many narrow levels cost the union a barrier of the whole GPU each. A level
+// takes about 14 us in the union and 8 in a team, an entry (a source's visit to a vertex)
+// 0.6 ns and 90, and a grid has about 2 sqrt(V) levels (a strip more, which favours teams
+// further: hence the quarter in their favour). As one graph / as teams, ms: 20 strips of
+// 300 x 5, 4 sources 6.0 / 2.9; 2 of 1500 x 4 19.5 / 13.1; 200 grids of 60 x 60, 4 sources 3.6 / 2.6;
+// 50 of 100 x 100 4.9 / 5.0; 10 of 200 x 200, 16 sources 10 / 57.
+static bool bc_teams_faster(sp_graph* g, int ngraphs, const std::vector<int32_t>& voff,
+                            const std::vector<int32_t>& soff) {
+  if (g->symmetric != 1 || g->max_out_deg < 0 || g->max_out_deg > bc::NARROW_DEG) return false;
+  double most = 0, all = 0, one = 0, levels = 0;  // teams: the longest graph, all together, us
+  for (int k = 0; k < ngraphs; ++k) {
+    const double n = voff[k + 1] - voff[k], visits = n * (soff[k + 1] - soff[k]), l = 2 * std::sqrt(n);
+    const double team = 8 * l + 0.09 * visits;
+    most = std::max(most, team);
+    all += team / (2 * num_sms());
+    one += 0.0006 * visits;
+    levels = std::max(levels, l);
+  }
+  return std::max(most, all) < 1.25 * (14 * levels + one);
+}
+}  // namespace sp
+
 extern "C" int sp_bc_graphs(sp_graph_h g, int32_t ngraphs, const int32_t* vertex_offset, const int32_t* source_offset,
                             const int32_t* sources, float* BC) {
   if (!g || ngraphs <= 0 || !vertex_offset || !source_offset || !BC) {
@@ -1685,7 +1709,7 @@ extern "C" int sp_bc_graphs(sp_graph_h g, int32_t ngraphs, const int32_t* vertex
   // 1.9 against 58. The union's state must fit;
   // a set bc.cluster asks for teams.
   const double state = (double)g->V * (std::min(smax, 64) <= 16 ? 16 : std::min(smax, 64) <= 32 ? 32 : 64) * 16;
-  if (g->bc_cluster <= 0 && nsrc > 0 && state <= bc::UNION_BYTES) {
+  if (g->bc_cluster <= 0 && nsrc > 0 && state <= bc::UNION_BYTES && !bc_teams_faster(g, ngraphs, voff, soff)) {
     int st = SP_OK;
     for (int width = std::min(smax, 64);; width = 16) {
       std::vector<int32_t> order, cols, boff{0};

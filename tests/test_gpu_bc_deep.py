@@ -48,3 +48,23 @@ def test_degree_borders(name, nsrc):
             rl, rs, _ = O.bfs_sigma(g.indexofNodes, g.edgeList, int(srcs[k]))
             assert np.array_equal(lv[k], rl)
             assert np.all(np.abs(sg[k] - rs) <= 1e-12 * rs)  # beyond 2^53 in the deep ones
+
+
+@pytest.mark.parametrize("shape,counts", [((20, 20), [3, 0, 16, 1]), ((150, 4), [40, 33, 2, 70]), ((70, 75), [16, 5, 9, 1])])
+def test_many_deep_graphs(shape, counts):
+    # small grids and strips: a CTA per graph where that is expected to be faster, and one
+    # union otherwise, against each graph by itself
+    one = G.grid(*shape)
+    n = one.V
+    u = np.repeat(np.arange(n, dtype=np.int32), np.diff(one.indexofNodes))
+    pairs = np.concatenate([np.stack([u, one.edgeList], 1) + n * k for k in range(4)])
+    union = from_pairs(4 * n, pairs)
+    srcs = [G.pick_sources(one, c, seed=k, min_out_degree=0) for k, c in enumerate(counts)]
+    voff = (n * np.arange(5)).astype(np.int32)
+    soff = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    ids = np.concatenate([s + n * k for k, s in enumerate(srcs)]).astype(np.int32)
+    with DeviceGraph.from_csr(union, with_weights=False) as dg:
+        out = dg.bc_graphs(voff, soff, ids).astype(np.float64)
+    for k in range(4):
+        ref = O.bc(one.indexofNodes, one.edgeList, srcs[k]) if counts[k] else np.zeros(n)
+        assert np.all(np.abs(out[n * k:n * k + n] - ref) <= 1e-5 * np.abs(ref) + 1e-9 * max(1.0, ref.max())), k
