@@ -203,11 +203,10 @@ __global__ void k_emap(int32_t V, int64_t E, const int32_t* __restrict__ off, co
   }
 }
 
-// *bad = 1 unless a[0 .. n) == b[0 .. n) (both 16-byte aligned). 16-byte loads, four of
-// each array in flight per thread: 31.4 M entries and 1 M offsets
+// Whether a[0 .. n) != b[0 .. n) in what this thread compares (both 16-byte aligned). 16-byte
+// loads, four of each array in flight per thread: 31.4 M entries and 1 M offsets
 // 123 us with one 4-byte pair at a time, 43 now.
-__global__ void __launch_bounds__(256) k_cmp(const int32_t* __restrict__ a, const int32_t* __restrict__ b, int64_t n,
-                                             int* __restrict__ bad) {
+__device__ __forceinline__ bool differ(const int32_t* __restrict__ a, const int32_t* __restrict__ b, int64_t n) {
   constexpr int U = 4;
   const int4* a4 = reinterpret_cast<const int4*>(a);
   const int4* b4 = reinterpret_cast<const int4*>(b);
@@ -227,7 +226,14 @@ __global__ void __launch_bounds__(256) k_cmp(const int32_t* __restrict__ a, cons
     if (diff) break;
   }
   if (me < n % 4) diff |= a[4 * n4 + me] ^ b[4 * n4 + me];
-  if (diff) *bad = 1;
+  return diff != 0;
+}
+
+// *bad = 1 unless both pairs of arrays are equal.
+__global__ void __launch_bounds__(256) k_cmp(const int32_t* __restrict__ a, const int32_t* __restrict__ b, int64_t n,
+                                             const int32_t* __restrict__ c, const int32_t* __restrict__ d, int64_t m,
+                                             int* __restrict__ bad) {
+  if (differ(a, b, n) || differ(c, d, m)) *bad = 1;
 }
 
 // CSR check in two coalesced passes (no warp ever walks a hub row alone).
@@ -405,16 +411,12 @@ int ensure_symmetry(sp_graph* g) {
   if (g->symmetric >= 0) return SP_OK;
   SP_TRY(ensure_reverse(g));
   cudaStream_t s = g->stream;
-  dbuf<int> bad;
-  SP_TRY(bad.alloc(1));
-  SP_CHECK_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
-  int grid = num_sms() * 4;
-  k_cmp<<<grid, 256, 0, s>>>(g->off.p, g->roff.p, (int64_t)g->V + 1, bad.p);
-  SP_CHECK_LAUNCH();
-  k_cmp<<<grid, 256, 0, s>>>(g->adj.p, g->radj.p, g->E, bad.p);
+  SP_TRY(g->flag.alloc(1));
+  SP_CHECK_CUDA(cudaMemsetAsync(g->flag.p, 0, sizeof(int), s));
+  k_cmp<<<num_sms() * 4, 256, 0, s>>>(g->off.p, g->roff.p, (int64_t)g->V + 1, g->adj.p, g->radj.p, g->E, g->flag.p);
   SP_CHECK_LAUNCH();
   int h = 0;
-  SP_TRY(copy_out(&h, bad.p, sizeof(int), s));
+  SP_TRY(copy_out(&h, g->flag.p, sizeof(int), s));
   g->symmetric = h ? 0 : 1;
   return SP_OK;
 }
@@ -572,6 +574,7 @@ int sp_graph_free(sp_graph_h g) {
   g->roff.release();
   g->radj.release();
   g->emap.release();
+  g->flag.release();
   if (g->own_stream && g->stream) cudaStreamDestroy(g->stream);
   delete g;
   return SP_OK;

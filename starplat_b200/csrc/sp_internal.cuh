@@ -155,6 +155,7 @@ struct sp_graph {
   sp::dbuf<int32_t> roff;  // rev_indexofNodes [V+1]
   sp::dbuf<int32_t> radj;  // srcList [E]
   sp::dbuf<int32_t> emap;  // edgeMap [E]: forward index of each reverse entry (built on demand)
+  sp::dbuf<int> flag;      // of the symmetry comparison: kept, as releasing memory waits for the device
   bool has_w = false;
   bool has_rev = false;
   int symmetric = -1;      // -1 unknown, 0/1

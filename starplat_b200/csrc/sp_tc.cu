@@ -996,9 +996,10 @@ static int order_part(sp_graph* g, int part, int nparts, dbuf<int32_t>& out, int
 }
 
 // Up to this many entries a symmetric graph of at most 65536 vertices is counted by
-// k_tc_bitmap_cta: both take a call's own time of about 30 us there (R-MAT 13 of edge
-// factor 8, 115 thousand entries: 33 against 30), and its plan is made in fewer launches
-// (a first call 223 against 272 us).
+// k_tc_bitmap_cta: both take a call's own time there (R-MAT 13 of edge factor 8, 111
+// thousand entries, 44 us). Above it the rank order is as fast on a first call, its plan
+// included, and faster on the next: R-MAT 13 of edge factor 16, 204 thousand entries, 227 and
+// 43 us against 228 and 54; ER 20,000 of degree 16 212 and 43 against 232 and 54.
 constexpr int64_t RANK_MIN_E = 1 << 17;
 
 // The triangles of part `part` of `nparts`. Symmetric graphs count in rank order

@@ -294,26 +294,42 @@ __global__ void __launch_bounds__(256) k_keep(int V, long long E, const int32_t*
     c.y = rank[row[1]] < ru[1];
     c.z = rank[row[2]] < ru[2];
     c.w = rank[row[3]] < ru[3];
-    *reinterpret_cast<uchar4*>(keep + i0) = c;  // past E: keep has room, and entry E is set afterwards
+    *reinterpret_cast<uchar4*>(keep + i0) = c;  // past E, where keep has room: 0
   });
+  if (E % 4 == 0 && blockIdx.x == 0 && threadIdx.x == 0) keep[E] = 0;  // the scan's last entry
 }
 
-// tasks of each anchor, by rank (entry V is 0)
-__global__ void k_task_counts(int V, const int32_t* __restrict__ off, const int32_t* __restrict__ pos,
-                              const int32_t* __restrict__ rank, int32_t* __restrict__ cnt) {
+// Per rank: its tasks as an anchor (x), the length of its row N+ (y), the row's vectors (z)
+// and its work items (w; none without a row of its own). Entry V is 0. The row's length is
+// what the anchor's part and a self-loop leave of the degree, so one scan gives every
+// position before the rows are sorted (searched for in the sorted rows, with scans of their
+// own, they took 30 us more of a first call).
+__global__ void k_row_sizes(int V, const int32_t* __restrict__ off, const int32_t* __restrict__ adj,
+                            const int32_t* __restrict__ pos, const int32_t* __restrict__ rank, int chunk,
+                            int4* __restrict__ size) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v <= V; v += gridDim.x * blockDim.x) {
-    if (v == V)
-      cnt[V] = 0;
-    else
-      cnt[rank[v]] = pos[off[v + 1]] - pos[off[v]];
+    if (v == V) {
+      size[V] = make_int4(0, 0, 0, 0);
+      continue;
+    }
+    const int b = off[v], e = off[v + 1], t = pos[e] - pos[b];
+    const int d = e - b - t - (in_list(adj + b, e - b, v) ? 1 : 0);
+    size[rank[v]] = make_int4(t, d, (d + 3) / 4, d > 0 ? (t + chunk - 1) / chunk : 0);
   }
 }
 
-// Task p of anchor v: tu[p] = u, ta[p] = v, id[p] = p (in ascending v).
+struct Plus4 {
+  __host__ __device__ __forceinline__ int4 operator()(const int4& a, const int4& b) const {
+    return make_int4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+  }
+};
+
+// Task p of anchor v: tu[p] = u, ta[p] = v, id[p] = p (in ascending v). After the last of them,
+// keys that sort behind every rank. start: the scanned sizes.
 __global__ void __launch_bounds__(256) k_emit(int V, long long E, const int32_t* __restrict__ off,
                                               const int32_t* __restrict__ adj, const int32_t* __restrict__ rank,
                                               const unsigned char* __restrict__ keep, const int32_t* __restrict__ pos,
-                                              const int32_t* __restrict__ tpos, int32_t* __restrict__ tu,
+                                              const int4* __restrict__ start, int mcap, int32_t* __restrict__ tu,
                                               int32_t* __restrict__ ta, int32_t* __restrict__ id) {
   edge_quads(V, E, off, adj, [&](long long i0, int n, const int (&row)[4], const int (&u)[4]) {
     const uchar4 c = *reinterpret_cast<const uchar4*>(keep + i0);
@@ -323,90 +339,53 @@ __global__ void __launch_bounds__(256) k_emit(int V, long long E, const int32_t*
     for (int k = 0; k < 4; ++k) {
       if (k >= n || !kc[k]) continue;
       const int r = rank[row[k]];
-      const int p = tpos[r] + (at - pos[off[row[k]]]);
+      const int p = start[r].x + (at - pos[off[row[k]]]);
       tu[p] = rank[u[k]];
       ta[p] = r;
       id[p] = p;
       ++at;
     }
   });
-}
-
-// tasks after the last: keys that sort behind every rank
-__global__ void k_pad(int mcap, const int32_t* __restrict__ m, int32_t* __restrict__ tu, int32_t* __restrict__ id) {
-  for (int p = *m + blockIdx.x * blockDim.x + threadIdx.x; p < mcap; p += gridDim.x * blockDim.x) {
+  for (int p = start[V].x + blockIdx.x * 256 + threadIdx.x; p < mcap; p += gridDim.x * 256) {
     tu[p] = -1;
     id[p] = p;
   }
 }
 
-// ooff[u] = the first of the *m sorted keys that is >= u
-__global__ void k_row_starts(int V, const int32_t* __restrict__ m, const int32_t* __restrict__ su,
-                             int32_t* __restrict__ ooff) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u <= V; u += gridDim.x * blockDim.x) {
-    int lo = 0, hi = *m;
-    while (lo < hi) {
-      const int c = (lo + hi) >> 1;
-      if (su[c] < u) lo = c + 1; else hi = c;
-    }
-    ooff[u] = lo;
-  }
-}
-
-// Per rank, packed for one scan: the vectors of its row N+(v) (low word), and its work
-// items as an anchor (high word; none without a list of its own). Entry V is 0.
-__global__ void k_counts(int V, const int32_t* __restrict__ ooff, const int32_t* __restrict__ tpos, int chunk,
-                         unsigned long long* __restrict__ cnt) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v <= V; v += gridDim.x * blockDim.x) {
-    unsigned long long c = 0;
-    if (v < V) {
-      const int d = ooff[v + 1] - ooff[v];
-      c = (unsigned long long)((d + 3) / 4);
-      if (d > 0) c |= (unsigned long long)((tpos[v + 1] - tpos[v] + chunk - 1) / chunk) << 32;
-    }
-    cnt[v] = c;
-  }
-}
-
 // The tasks stably sorted by u are the rows N+(u), each ascending: entry e of the sorted
 // order is task sp[e], whose anchor is the element, and whose prefix is what stands
-// before it in its row. Low word of vpos[u] = the row's first vector. A prefix has at most
+// before it in its row. A prefix has at most
 // sqrt(2 m) < 2^16 elements, so its vectors go to their task as 2 bytes: the scattered
 // writes stay in L2 (whole 8-byte tasks: 0.68 ms for 16.8 M, now 0.24 and 0.09 in k_tasks).
-__global__ void k_rows(const int32_t* __restrict__ mp, const int32_t* __restrict__ su, const int32_t* __restrict__ sp,
-                       const int32_t* __restrict__ ta, const int32_t* __restrict__ ooff,
-                       const unsigned long long* __restrict__ vpos, int32_t* __restrict__ oadj,
+__global__ void k_rows(int V, const int32_t* __restrict__ su, const int32_t* __restrict__ sp,
+                       const int32_t* __restrict__ ta, const int4* __restrict__ start, int32_t* __restrict__ oadj,
                        unsigned short* __restrict__ nvec) {
-  const int m = *mp;
+  const int m = start[V].x;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
-    const int p = sp[e], u = su[e], before = e - ooff[u];
-    long long at = 4ll * (int)vpos[u] + before;
+    const int p = sp[e], u = su[e];
+    const int4 s = start[u];
+    const int before = e - s.y;
+    long long at = 4ll * s.z + before;
     oadj[at] = ta[p];
-    if (e + 1 == ooff[u + 1])
+    if (e + 1 == start[u + 1].y)
       while (++at & 3) oadj[at] = -1;
     nvec[p] = (unsigned short)((before + 3) / 4);
   }
 }
 
-__global__ void k_tasks(const int32_t* __restrict__ mp, const int32_t* __restrict__ tu,
-                        const unsigned long long* __restrict__ vpos, const unsigned short* __restrict__ nvec,
-                        int2* __restrict__ tasks) {
-  const int m = *mp;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x)
-    tasks[p] = make_int2((int)vpos[tu[p]], nvec[p]);
-}
-
-// The work items of every anchor, and their number.
-__global__ void k_items(int V, const int32_t* __restrict__ ooff, const unsigned long long* __restrict__ vpos,
-                        const int32_t* __restrict__ tpos, int chunk, int4* __restrict__ items,
-                        int32_t* __restrict__ itemv, int32_t* __restrict__ n_items) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    const int end = (int)(vpos[v + 1] >> 32);
-    for (int k = (int)(vpos[v] >> 32), t = tpos[v]; k < end; ++k, t += chunk) {
-      items[k] = make_int4(t, min(chunk, tpos[v + 1] - t), (int)vpos[v], ooff[v + 1] - ooff[v]);
+// The tasks, the work items of every anchor, and their number.
+__global__ void k_tasks(int V, const int32_t* __restrict__ tu, const int4* __restrict__ start,
+                        const unsigned short* __restrict__ nvec, int chunk, int2* __restrict__ tasks,
+                        int4* __restrict__ items, int32_t* __restrict__ itemv, int32_t* __restrict__ n_items) {
+  const int m = start[V].x, t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  for (int p = t0; p < m; p += nt) tasks[p] = make_int2(start[tu[p]].z, nvec[p]);
+  for (int v = t0; v < V; v += nt) {
+    const int4 s = start[v], e = start[v + 1];
+    for (int k = s.w, t = s.x; k < e.w; ++k, t += chunk) {
+      items[k] = make_int4(t, min(chunk, e.x - t), s.z, e.y - s.y);
       itemv[k] = v;
     }
-    if (v == V - 1) *n_items = end;
+    if (v == V - 1) *n_items = e.w;
   }
 }
 
@@ -446,29 +425,25 @@ inline int build(sp_graph* g, Plan& P) {
   // what the build alone needs, in one block
   Arena tmp;
   dspan<unsigned> key, skey;
-  dspan<int32_t> id, rank, pos, cnt, ooff, tpos, ta, tid, su, sp;
-  dspan<unsigned long long> both, vpos;
+  dspan<int32_t> id, rank, pos, ta, tid, su, sp;
+  dspan<int4> size, start;
   dspan<unsigned char> keep, cubt;
   dspan<unsigned short> nvec;
-  size_t t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0;
+  size_t t1 = 0, t2 = 0, t3 = 0, t4 = 0;
   SP_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t1, (unsigned*)nullptr, (unsigned*)nullptr,
                                                 (int32_t*)nullptr, (int32_t*)nullptr, V, 0, dbits, s));
   SP_CHECK_CUDA(cub::DeviceScan::ExclusiveScan(nullptr, t2, (unsigned char*)nullptr, (int32_t*)nullptr, Plus{},
                                                (int32_t)0, (int)(E + 1), s));
   SP_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t3, (int32_t*)nullptr, (int32_t*)nullptr, (int32_t*)nullptr,
                                                 (int32_t*)nullptr, (int)mcap, 0, vbits, s));
-  SP_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t4, (int32_t*)nullptr, (int32_t*)nullptr, V + 1, s));
-  SP_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t5, (unsigned long long*)nullptr, (unsigned long long*)nullptr,
-                                              V + 1, s));
+  SP_CHECK_CUDA(cub::DeviceScan::ExclusiveScan(nullptr, t4, (int4*)nullptr, (int4*)nullptr, Plus4{},
+                                               make_int4(0, 0, 0, 0), V + 1, s));
   tmp.want(key, V);
   tmp.want(skey, V);
   tmp.want(id, V);
   tmp.want(rank, V);
-  tmp.want(cnt, V + 1);
-  tmp.want(ooff, V + 1);
-  tmp.want(tpos, V + 1);
-  tmp.want(both, V + 1);
-  tmp.want(vpos, V + 1);
+  tmp.want(size, V + 1);
+  tmp.want(start, V + 1);
   tmp.want(keep, E + 4);
   tmp.want(nvec, mcap);
   tmp.want(pos, E + 1);
@@ -476,7 +451,7 @@ inline int build(sp_graph* g, Plan& P) {
   tmp.want(tid, mcap);
   tmp.want(su, mcap);
   tmp.want(sp, mcap);
-  tmp.want(cubt, std::max({t1, t2, t3, t4, t5}));
+  tmp.want(cubt, std::max({t1, t2, t3, t4}));
   SP_TRY(tmp.commit());
   P.mem.want(P.order, V);
   P.mem.want(P.oadj, (size_t)mcap + 3 * (size_t)std::min<long long>(V, mcap));
@@ -502,39 +477,27 @@ inline int build(sp_graph* g, Plan& P) {
   if (E > 0) {
     k_keep<<<eg, 256, 0, s>>>(V, E, g->off.p, g->adj.p, rank.p, keep.p);
     SP_CHECK_LAUNCH();
+  } else {
+    SP_CHECK_CUDA(cudaMemsetAsync(keep.p, 0, 1, s));
   }
-  SP_CHECK_CUDA(cudaMemsetAsync(keep.p + E, 0, 1, s));
   SP_CHECK_CUDA(cub::DeviceScan::ExclusiveScan(cubt.p, t2, keep.p, pos.p, Plus{}, (int32_t)0, (int)(E + 1), s));
-  k_task_counts<<<vg, 256, 0, s>>>(V, g->off.p, pos.p, rank.p, cnt.p);
+  k_row_sizes<<<vg, 256, 0, s>>>(V, g->off.p, g->adj.p, pos.p, rank.p, chunk, size.p);
   SP_CHECK_LAUNCH();
-  SP_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(cubt.p, t4, cnt.p, tpos.p, V + 1, s));
-  const int32_t* m = tpos.p + V;  // the tasks: mcap, less the self-loops' entries
-  const int mg = (int)std::max<long long>(1, std::min<long long>((mcap + 255) / 256, num_sms() * 8));
+  SP_CHECK_CUDA(cub::DeviceScan::ExclusiveScan(cubt.p, t4, size.p, start.p, Plus4{}, make_int4(0, 0, 0, 0), V + 1, s));
+  // the tasks: mcap, less the self-loops' entries
+  const int mg = (int)std::max<long long>(1, std::min<long long>((std::max<long long>(mcap, V) + 255) / 256, num_sms() * 8));
   if (mcap > 0) {
-    k_emit<<<eg, 256, 0, s>>>(V, E, g->off.p, g->adj.p, rank.p, keep.p, pos.p, tpos.p, P.tu.p, ta.p, tid.p);
-    SP_CHECK_LAUNCH();
-    k_pad<<<std::min(mg, num_sms()), 256, 0, s>>>((int)mcap, m, P.tu.p, tid.p);
+    k_emit<<<eg, 256, 0, s>>>(V, E, g->off.p, g->adj.p, rank.p, keep.p, pos.p, start.p, (int)mcap, P.tu.p, ta.p,
+                              tid.p);
     SP_CHECK_LAUNCH();
     SP_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(cubt.p, t3, P.tu.p, su.p, tid.p, sp.p, (int)mcap, 0, vbits, s));
+    k_rows<<<mg, 256, 0, s>>>(V, su.p, sp.p, ta.p, start.p, P.oadj.p, nvec.p);
+    SP_CHECK_LAUNCH();
   }
-  k_row_starts<<<vg, 256, 0, s>>>(V, m, su.p, ooff.p);
+  k_tasks<<<mg, 256, 0, s>>>(V, P.tu.p, start.p, nvec.p, chunk, P.tasks.p, P.items.p, P.itemv.p,
+                             (int32_t*)(P.out.p + OUT_ITEMS));
   SP_CHECK_LAUNCH();
-  k_counts<<<vg, 256, 0, s>>>(V, ooff.p, tpos.p, chunk, both.p);
-  SP_CHECK_LAUNCH();
-  SP_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(cubt.p, t5, both.p, vpos.p, V + 1, s));
-  if (mcap > 0) {
-    k_rows<<<mg, 256, 0, s>>>(m, su.p, sp.p, ta.p, ooff.p, vpos.p, P.oadj.p, nvec.p);
-    SP_CHECK_LAUNCH();
-    k_tasks<<<mg, 256, 0, s>>>(m, P.tu.p, vpos.p, nvec.p, P.tasks.p);
-    SP_CHECK_LAUNCH();
-  }
-  if (V > 0) {
-    k_items<<<vg, 256, 0, s>>>(V, ooff.p, vpos.p, tpos.p, chunk, P.items.p, P.itemv.p, (int32_t*)(P.out.p + OUT_ITEMS));
-    SP_CHECK_LAUNCH();
-  } else {
-    SP_CHECK_CUDA(cudaMemsetAsync(P.out.p + OUT_ITEMS, 0, sizeof(unsigned long long), s));
-  }
-  g_launches += 5;  // the scans and sorts
+  g_launches += 4;  // the scans and sorts
   P.items_max = (int)std::min<long long>(imax, INT32_MAX);
   P.built = true;
   return SP_OK;
