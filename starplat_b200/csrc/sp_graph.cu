@@ -236,6 +236,38 @@ __global__ void __launch_bounds__(256) k_cmp(const int32_t* __restrict__ a, cons
   if (differ(a, b, n) || differ(c, d, m)) *bad = 1;
 }
 
+// *bad = 1 unless every entry u -> v has its opposite. Edge-parallel in tiles of EDGE_TILE
+// entries, a binary search in v's row each; a block ends where one is missing.
+__global__ void __launch_bounds__(256) k_opposites(int32_t V, int64_t E, const int32_t* __restrict__ off,
+                                                   const int32_t* __restrict__ adj, int* bad) {
+  __shared__ int s_v[3];
+  for (long long t0 = (long long)blockIdx.x * EDGE_TILE; t0 < E; t0 += (long long)gridDim.x * EDGE_TILE) {
+    const long long t1 = t0 + EDGE_TILE < E ? t0 + EDGE_TILE : E;
+    if (threadIdx.x < 2) s_v[threadIdx.x] = edge_source(off, 0, V, threadIdx.x == 0 ? t0 : t1 - 1);
+    if (threadIdx.x == 2) s_v[2] = *(volatile int*)bad;
+    __syncthreads();
+    if (s_v[2]) return;  // the same for the block
+    const int vlo = s_v[0], vhi = s_v[1];
+    for (long long e0 = t0; e0 < t1; e0 += blockDim.x) {
+      const long long e = e0 + threadIdx.x;
+      bool miss = false;
+      if (e < t1) {
+        const int u = edge_source(off, vlo, vhi + 1, e), v = adj[e], end = off[v + 1];
+        int lo = off[v], hi = end;
+        while (lo < hi) {
+          const int m = (lo + hi) >> 1;
+          if (adj[m] < u) lo = m + 1; else hi = m;
+        }
+        miss = lo == end || adj[lo] != u;
+      }
+      if (__syncthreads_or(miss)) {  // a directed graph ends here, in every block
+        if (threadIdx.x == 0) *bad = 1;
+        return;
+      }
+    }
+  }
+}
+
 // CSR check in two coalesced passes (no warp ever walks a hub row alone).
 // res[0] = flags: 1 offsets not monotone within [0, E] (or off[0] != 0, off[V] != E),
 // 2 an id outside [0, V), 4 a row not strictly increasing (unsorted or duplicate);
@@ -346,6 +378,13 @@ int ensure_reverse(sp_graph* g) {
   const int64_t E = g->E;
   SP_TRY(g->roff.alloc((size_t)V + 1));
   SP_TRY(g->radj.alloc(E));
+  if (g->symmetric == 1) {
+    SP_CHECK_CUDA(cudaMemcpyAsync(g->roff.p, g->off.p, sizeof(int32_t) * ((size_t)V + 1), cudaMemcpyDeviceToDevice, s));
+    if (E > 0) SP_CHECK_CUDA(cudaMemcpyAsync(g->radj.p, g->adj.p, 4 * (size_t)E, cudaMemcpyDeviceToDevice, s));
+    SP_CHECK_CUDA(cudaStreamSynchronize(s));
+    g->has_rev = true;
+    return SP_OK;
+  }
   int bits = 1;
   while (bits < 31 && (1 << bits) < V) ++bits;
   size_t t_sort = 0;
@@ -407,15 +446,38 @@ int ensure_emap(sp_graph* g) {
   return SP_OK;
 }
 
+// Up to this many entries a graph without in-edges is tested for symmetry by looking for every
+// entry's opposite: to learn it takes 57 us instead of 134 on R-MAT 14 (329 thousand
+// entries), 265 instead of 366 on R-MAT 18 (7.6 M), 372 instead of 652 on ER 2^20 (16.8 M), and
+// 1,066 instead of 1,009 on R-MAT 20 (31 M), where building the in-edges and comparing is
+// faster. A directed graph loses 4 to 12 us before its in-edges are built.
+constexpr int64_t OPPOSITES_MAX_E = 1 << 24;
+
 int ensure_symmetry(sp_graph* g) {
   if (g->symmetric >= 0) return SP_OK;
-  SP_TRY(ensure_reverse(g));
   cudaStream_t s = g->stream;
   SP_TRY(g->flag.alloc(1));
   SP_CHECK_CUDA(cudaMemsetAsync(g->flag.p, 0, sizeof(int), s));
+  int h = 0;
+  if (!g->has_rev && g->E <= OPPOSITES_MAX_E) {
+    if (g->E > 0) {
+      const int tiles = (int)std::min<int64_t>((g->E + EDGE_TILE - 1) / EDGE_TILE, num_sms() * 8);
+      k_opposites<<<tiles, 256, 0, s>>>(g->V, g->E, g->off.p, g->adj.p, g->flag.p);
+      SP_CHECK_LAUNCH();
+      SP_TRY(copy_out(&h, g->flag.p, sizeof(int), s));
+    }
+    if (!h) {
+      g->symmetric = 1;
+      return SP_OK;
+    }
+  }
+  SP_TRY(ensure_reverse(g));
+  if (h) {
+    g->symmetric = 0;
+    return SP_OK;
+  }
   k_cmp<<<num_sms() * 4, 256, 0, s>>>(g->off.p, g->roff.p, (int64_t)g->V + 1, g->adj.p, g->radj.p, g->E, g->flag.p);
   SP_CHECK_LAUNCH();
-  int h = 0;
   SP_TRY(copy_out(&h, g->flag.p, sizeof(int), s));
   g->symmetric = h ? 0 : 1;
   return SP_OK;
