@@ -627,18 +627,41 @@ __global__ void k_tot(int n, const int32_t* __restrict__ comm, const double* __r
 // smaller vertex is not looked up. 113 us before (whole, rows found by a search over the
 // lanes); now 96 at 3 steps and 6 CTAs an SM, 105 at 4 and 6, 110 at 2 and 8, 144 at 6 and 4:
 // latency of adj (read from DRAM each time) and comm bounds it.
-constexpr int INTERNAL_CTAS = 6;
-template <bool HALF>
+// LONG (a graph that may have them): rows of more than LONG_ROW edges are left to the CTA, whose
+// warps take their pieces of 32 * LU edges in turn, in a fixed order; LONG_CAP a warp, and
+// what it has beyond those by itself. Neighbouring groups of 32 vertices go to different CTAs,
+// as an R-MAT graph's hubs are neighbours. While a warp walked its 32 vertices' rows alone,
+// 32 hubs held up the rest: the whole Louvain of R-MAT 17 took 29.9 ms, now 19.5 (22.9 with
+// neighbouring groups in one CTA).
+constexpr int INTERNAL_CTAS = 6, LONG_ROW = 512, LONG_CAP = 96, LU = 8;
+template <bool HALF, bool LONG>
 __global__ void __launch_bounds__(THREADS, INTERNAL_CTAS) k_internal(Level L, const int32_t* __restrict__ comm, double W,
                                                       double* q) {
   constexpr int U = 3;
   __shared__ double s_red[THREADS / 32];
   __shared__ int s_row[THREADS / 32][32], s_com[THREADS / 32][32], s_v[HALF ? THREADS / 32 : 1][32];
+  __shared__ int s_long[LONG ? THREADS / 32 : 1][LONG_CAP], s_longs[THREADS / 32];  // per warp: the rows left to the CTA
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned le = FULL >> (31 - lane);
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  const int gw = LONG ? wid * gridDim.x + blockIdx.x : (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nw = gridDim.x * (THREADS / 32);
   double acc = 0;
+  int longs = 0;  // of this warp
+  auto row = [&](int me, int part, int parts) {
+    const int rb = L.off[me], re = L.off[me + 1], cm = comm[me];
+    for (int k0 = rb + 32 * LU * part + lane; k0 < re; k0 += 32 * LU * parts) {
+      int u[LU];
+#pragma unroll
+      for (int q = 0; q < LU; ++q) {
+        u[q] = k0 + 32 * q < re ? L.adj[k0 + 32 * q] : -1;
+        if (HALF && u[q] < me) u[q] = -1;
+      }
+#pragma unroll
+      for (int q = 0; q < LU; ++q)
+        if (u[q] >= 0 && comm[u[q]] == cm) acc += HALF ? (u[q] > me ? 2.0 : 1.0) : L.unit ? 1.0 : L.w[k0 + 32 * q];
+    }
+  };
   for (int base = gw * 32; base < L.n; base += nw * 32) {
     const int v = base + lane;
     int b = 0, d = 0, cv = -1;
@@ -647,6 +670,16 @@ __global__ void __launch_bounds__(THREADS, INTERNAL_CTAS) k_internal(Level L, co
       d = L.off[v + 1] - b;
       cv = comm[v];
       acc += L.sl[v];
+    }
+    if (LONG) {
+      const unsigned lng = __ballot_sync(FULL, d > LONG_ROW);
+      if (d > LONG_ROW) {
+        const int k = longs + __popc(lng & (le >> 1));
+        if (k < LONG_CAP) s_long[wid][k] = v;
+        d = 0;
+      }
+      for (unsigned m = lng; m; m &= m - 1)
+        if (longs++ >= LONG_CAP) row(base + __ffs(m) - 1, 0, 1);
     }
     int inc = d;
 #pragma unroll
@@ -698,6 +731,12 @@ __global__ void __launch_bounds__(THREADS, INTERNAL_CTAS) k_internal(Level L, co
         if (u[q] >= 0 && comm[u[q]] == cq[q]) acc += wq[q];
     }
     __syncwarp();
+  }
+  if (LONG) {
+    if (lane == 0) s_longs[wid] = min(longs, LONG_CAP);
+    __syncthreads();
+    for (int w = 0; w < THREADS / 32; ++w)
+      for (int k = 0; k < s_longs[w]; ++k) row(s_long[w][k], wid, THREADS / 32);
   }
   acc = block_sum<THREADS>(acc, s_red);
   if (threadIdx.x == 0) q[blockIdx.x] = acc / W;
@@ -861,14 +900,13 @@ int read_int(const int* d, int* h, cudaStream_t s) { return copy_out(h, d, sizeo
 
 }  // namespace
 
-static int lv_modularity(LvPlan* p, const lv::Level& L, double W, bool half, cudaStream_t s, double* q) {
+static int lv_modularity(LvPlan* p, const lv::Level& L, double W, bool half, bool longs, cudaStream_t s, double* q) {
   const int n = L.n;
   const int g = num_sms() * lv::INTERNAL_CTAS;
   SP_TRY(p->qpart.alloc(2 * (size_t)g));
-  if (half)
-    lv::k_internal<true><<<g, lv::THREADS, 0, s>>>(L, p->comm.p, W, p->qpart.p);
-  else
-    lv::k_internal<false><<<g, lv::THREADS, 0, s>>>(L, p->comm.p, W, p->qpart.p);
+  auto internal = half ? longs ? lv::k_internal<true, true> : lv::k_internal<true, false>
+                       : longs ? lv::k_internal<false, true> : lv::k_internal<false, false>;
+  internal<<<g, lv::THREADS, 0, s>>>(L, p->comm.p, W, p->qpart.p);
   SP_CHECK_LAUNCH();
   lv::k_q<<<g, lv::THREADS, 0, s>>>(n, p->tot.p, W, p->qpart.p + g);
   SP_CHECK_LAUNCH();
@@ -1133,7 +1171,9 @@ extern "C" int sp_louvain(sp_graph_h g, const float* weight, double threshold, i
     }
     SP_TRY(lv_recount(p, n, s));
     double qlev0 = 0;
-    SP_TRY(lv_modularity(p, L, W, half && levels == 0, s, &qlev0));
+    // rows of the input graph are known; a coarser graph's are not read back
+    const bool longs = levels > 0 || g->max_out_deg < 0 || g->max_out_deg > lv::LONG_ROW;
+    SP_TRY(lv_modularity(p, L, W, half && levels == 0, longs, s, &qlev0));
     if (first) qcur = qlev0;
     first = false;
     // kernel variant of this level, chosen on the device (forced, learned, or the
@@ -1227,7 +1267,7 @@ extern "C" int sp_louvain(sp_graph_h g, const float* weight, double threshold, i
       }
       qold = qnew;
       ++total_sweeps;
-      SP_TRY(lv_modularity(p, L, W, half && levels == 0, s, &qnew));
+      SP_TRY(lv_modularity(p, L, W, half && levels == 0, longs, s, &qnew));
       if (!(qnew - qold > threshold)) break;
     }
     if (ev0) {
