@@ -506,7 +506,11 @@ __global__ void __launch_bounds__(THREADS, 8) k_phase(IterArgs a, const float* _
 // R-MAT 22 11.6 against 12.8 (8 CTAs an SM) to 18.8 (3). So it runs up to RUN_MAX_E in-edges
 // (ER 300,000: 4.8 M, 422 -> 358 us), or RUN_MAX_LONG_E where rows are split in chunks.
 constexpr int RUN_CTAS = 4;
-constexpr int64_t RUN_MAX_E = 6000000, RUN_MAX_LONG_E = 1500000;
+// Where beta asks for all max_iter iterations there are no idle launches to save, so only up
+// to RUN_ALL_E: 100 iterations of R-MAT 100,000 (1.4 M) 1.63 ms against 1.65, of ER 200,000
+// (3.2 M) 1.22 against 1.17 (a first call 1.58 against 1.75), of ER 370,000 (5.9 M) 2.40
+// against 2.10 (2.83 against 2.79).
+constexpr int64_t RUN_MAX_E = 6000000, RUN_MAX_LONG_E = 1500000, RUN_ALL_E = 4000000;
 struct RunBufs {
   float* pr[2];
   float* con[2];
@@ -1382,7 +1386,9 @@ static int pr_tuned(sp_graph* g, float beta, float delta, int32_t maxIter, float
   const RunFn run = runs[sh][gh][vec];
   const int exec_key = sh | (vec << 2) | (l1_hot << 3);
   // one launch for all iterations where the launches would cost more than it does
-  const bool whole = !a.two_phase && g->E <= (p->n_chunks[1] ? pr::RUN_MAX_LONG_E : pr::RUN_MAX_E);
+  const int64_t whole_max = std::min(p->n_chunks[1] ? pr::RUN_MAX_LONG_E : pr::RUN_MAX_E,
+                                     beta > 0 ? pr::RUN_MAX_E : pr::RUN_ALL_E);
+  const bool whole = !a.two_phase && g->E <= whole_max;
   const void* fn = whole ? (const void*)run : (const void*)ph1;
   SP_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, pr::THREADS, 0));
   const int grid = std::max(1, std::min(num_sms() * 32, num_sms() * std::max(1, per_sm)));
@@ -1442,11 +1448,11 @@ static int pr_tuned(sp_graph* g, float beta, float delta, int32_t maxIter, float
   int queued = 0;  // iterations launched
   if (!cached && !repeat) {
     // first call with these settings: launch directly (no capture and instantiation
-    // before the first kernel runs); a call that repeats them captures the graph. The stop
-    // test is read back after 16, 24, 36 ... iterations: a launch that finds the run ended
+    // before the first kernel runs); a call that repeats them captures the graph. Where beta
+    // lets a run end early the stop test is read back after 16, 24, 36 ... iterations: a launch that finds the run ended
     // takes 3 us (R-MAT 20 after a batch of updates: 77 of 100, 227 us of 2.8 ms), a read
     // about 15.
-    for (int to = 16; queued < n_iter; to += to / 2) {
+    for (int to = beta > 0 ? 16 : n_iter; queued < n_iter; to += to / 2) {
       const int end = std::min(n_iter, to);
       enqueue(s, queued, end);
       SP_CHECK_LAUNCH();
