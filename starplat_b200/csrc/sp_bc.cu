@@ -1176,8 +1176,8 @@ static int bc_gather(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch, in
   // the caller falls back to).
   const double E = (double)g->E;
   while (16 * (E / W.hub_chunk + E / W.hub_deg) > (double)(1 << 30)) {  // counts stay below 2^31
-    W.hub_deg *= 2;
-    W.hub_chunk *= 2;
+    W.hub_deg = W.hub_deg < (1 << 29) ? 2 * W.hub_deg : 1 << 30;  // both knobs go up to 2^30
+    W.hub_chunk = W.hub_chunk < (1 << 29) ? 2 * W.hub_chunk : 1 << 30;
   }
   const double copies = width > 16 ? 4 : width;
   const bool sym = g->symmetric == 1;

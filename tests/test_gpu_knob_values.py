@@ -67,3 +67,24 @@ def test_bc_knobs_read_back_what_runs():
         a = dg.bc_graphs(v, np.array([0, 5], np.int32), s)
         dg.tune_set("bc.cluster", dg.tune_get("bc.cluster"))
         assert np.array_equal(a, dg.bc_graphs(v, np.array([0, 5], np.int32), s))
+
+
+def test_bc_widest_and_narrowest_pieces_on_a_large_graph():
+    # 70 M entries at the largest hub_deg and the smallest hub_chunk: the pieces' size is
+    # raised until their number fits, without running over
+    import torch
+
+    V = 1 << 18
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    a, b = torch.randint(V, (2, 38_000_000), generator=gen, device="cuda")
+    key = torch.unique(torch.cat([a * V + b, b * V + a]))
+    off = torch.searchsorted(key, torch.arange(V + 1, device="cuda") * V).to(torch.int32)
+    adj = (key % V).to(torch.int32)
+    assert adj.numel() > 1 << 26
+    del a, b, key
+    with DeviceGraph(off, adj, None, off, adj) as dg:
+        ref = dg.bc(np.array([3], np.int32)).astype(np.float64)
+        dg.tune_set("bc.hub_deg", 1 << 30)
+        dg.tune_set("bc.hub_chunk", 1)
+        out = dg.bc(np.array([3], np.int32)).astype(np.float64)
+    assert np.all(np.abs(out - ref) <= 1e-6 * np.abs(ref))
