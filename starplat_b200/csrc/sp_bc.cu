@@ -58,6 +58,12 @@ constexpr int HUB_CHUNK = 64;
 constexpr int WIDE_HUB_DEG = 256, WIDE_HUB_CHUNK = 128;
 constexpr double WIDE_E = 12e6;
 constexpr int NARROW_DEG = 8;
+// Levels and path counts on a graph without in-edges: a first call of up to this many entries
+// times sources pushes, as the in-edges that the gather form needs cost more than it gains.
+// One source, first call pushing / gathering: directed R-MAT 14 (175 thousand entries) 0.27 / 0.41
+// ms, 17 (1.9 M) 0.45 / 0.58, R-MAT 17 (3.6 M) 0.46 / 0.50; 16 sources, directed 14 0.44 / 0.51,
+// 17 0.95 / 0.92, R-MAT 17 1.16 / 0.90.
+constexpr int64_t PUSH_MAX_E = 8000000;
 constexpr int CLUSTER_DEFAULT = 1;  // CTAs per graph in the many-graphs form (bc.cluster)
 // Successors whose loads are in flight together in the backward sweep (measured when
 // each successor cost a sigma and a delta load),
@@ -1012,6 +1018,7 @@ struct BcPlan {
   // gather form: the pieces and split entries of the level lists
   dbuf<int4> piece, rpiece;
   dbuf<int32_t> hub, rhub, plo;
+  bool levels_ran = false;  // levels and path counts were asked for before
   // learned variant inputs (vstat < 0: not yet) and the choice for var_nsrc sources
   int vstat = -1;
   int64_t vmax = 0, vsq = 0, vrows[4] = {}, vedges[4] = {};
@@ -1274,10 +1281,10 @@ static int bc_gather(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch, in
 }
 
 // The push / pull form, whose forward direction per level is chosen by the knob bc.dir or
-// the level model; bc.dir = 0 (the default without a model) takes the gather form.
+// the level model; bc.dir = 0 (the default without a model) takes the gather form, unless push.
 static int bc_grid(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch_hint, int32_t* lvl_out = nullptr,
-                   double* sig_out = nullptr) {
-  if (bc_direction(g) == 0) {
+                   double* sig_out = nullptr, bool push = false) {
+  if (bc_direction(g) == 0 && !push) {
     const int batch = std::max(1, std::min(std::min(batch_hint, 64), nsrc));
     return bc_gather(g, d_srcs, nsrc, batch, batch, 1 << 14, lvl_out, sig_out);
   }
@@ -1760,7 +1767,9 @@ int bc_levels(sp_graph* g, const int32_t* d_srcs, int nsrc, int32_t* lvl_out, do
     return SP_OK;
   };
   SP_TRY(clear());
-  int st = bc_grid(g, d_srcs, nsrc, 64, lvl_out, sig_out);
+  const bool push = !g->bc->levels_ran && !g->has_rev && g->symmetric < 0 && g->E * nsrc <= bc::PUSH_MAX_E;
+  g->bc->levels_ran = true;
+  int st = bc_grid(g, d_srcs, nsrc, 64, lvl_out, sig_out, push);
   if (st != SP_ERR_UNSUPPORTED || nsrc <= 16) return st;
   SP_TRY(clear());
   for (int k = 0; k < nsrc; k += 16)

@@ -68,3 +68,23 @@ def test_many_deep_graphs(shape, counts):
     for k in range(4):
         ref = O.bc(one.indexofNodes, one.edgeList, srcs[k]) if counts[k] else np.zeros(n)
         assert np.all(np.abs(out[n * k:n * k + n] - ref) <= 1e-5 * np.abs(ref) + 1e-9 * max(1.0, ref.max())), k
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("nsrc", [1, 16, 64])
+def test_levels_without_in_edges(directed, nsrc):
+    # a first call of few sources needs no in-edges, later ones and larger calls (8 M entries
+    # times sources) make them: the same levels and path counts
+    g = G.rmat(15, 8, seed=5, directed=directed)
+    assert (g.E * nsrc > 8_000_000) == (nsrc == 64)
+    srcs = G.pick_sources(g, nsrc, seed=2, min_out_degree=0)
+    with DeviceGraph(g.indexofNodes, g.edgeList, None, None, None) as dg:
+        runs = [dg.bfs_sigma(srcs) for _ in range(3)]
+        cc = [dg.closeness_unweighted(srcs) for _ in range(2)]
+    with DeviceGraph(g.indexofNodes, g.edgeList, None, None, None) as dg:
+        cc.append(dg.closeness_unweighted(srcs))
+    for k in range(0, nsrc, 5):
+        rl, rs, _ = O.bfs_sigma(g.indexofNodes, g.edgeList, int(srcs[k]))
+        for lv, sg in runs:
+            assert np.array_equal(lv[k], rl) and np.array_equal(sg[k], rs)
+    assert np.array_equal(cc[0], cc[1]) and np.array_equal(cc[0], cc[2])
