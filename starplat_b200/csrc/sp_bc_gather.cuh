@@ -278,6 +278,7 @@ __device__ __noinline__ void sweep(const Gather& G, const int32_t* __restrict__ 
                                    bool discover, int gw, int nw, Picked& pk) {
   const unsigned FULL = 0xffffffffu;
   constexpr int LPE = SW / 4, EPS = 32 / LPE;
+  if (gw * EPS >= e - b + (p1 - p0)) return;  // no item for this warp
   const int lane = threadIdx.x & 31, g = lane / LPE, sl = lane % LPE;
   const unsigned lt = (1u << lane) - 1u;
   const unsigned group = (LPE == 32 ? FULL : (1u << (LPE & 31)) - 1u) << (g * LPE);
