@@ -48,7 +48,6 @@ namespace sp {
 namespace lv {
 constexpr int THREADS = 256;
 constexpr int WARP_DEG = 64;
-
 constexpr int CTA_SLOTS_MAX = 16384;
 constexpr int EMPTY = -1;
 

@@ -719,14 +719,16 @@ static int build_tc_plan(sp_graph* g) {
   if (!g->tc) g->tc = new TcPlan();
   TcPlan* p = g->tc;
   cudaStream_t s = g->stream;
-  auto fail = [&](int st) { return st; };  // what was built is kept; a later call builds again
-  int st;
-  if ((st = p->heavy.alloc(g->V)) || (st = p->ctr.alloc(2)) || (st = p->total.alloc(1))) return fail(st);
+  // (what an error leaves built is kept; a later call builds again)
+  SP_TRY(p->heavy.alloc(g->V));
+  SP_TRY(p->ctr.alloc(2));
+  SP_TRY(p->total.alloc(1));
   if (g->symmetric == 1) {
-    if ((st = p->ooff.alloc(g->V + 1))) return fail(st);
+    SP_TRY(p->ooff.alloc(g->V + 1));
     const long long E = g->E;
     dbuf<int32_t> keep, pos;
-    if ((st = keep.alloc(E + 1)) || (st = pos.alloc(E + 1))) return fail(st);
+    SP_TRY(keep.alloc(E + 1));
+    SP_TRY(pos.alloc(E + 1));
     cudaMemsetAsync(keep.p + E, 0, sizeof(int32_t), s);
     if (E > 0) {
       tc::k_orient_flag<<<num_sms() * 8, 256, 0, s>>>(g->V, E, g->off.p, g->adj.p, keep.p);
@@ -735,21 +737,21 @@ static int build_tc_plan(sp_graph* g) {
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, keep.p, pos.p, (int)(E + 1), s);
     dbuf<unsigned char> tmp;
-    if ((st = tmp.alloc(tb))) return fail(st);
+    SP_TRY(tmp.alloc(tb));
     cub::DeviceScan::ExclusiveSum(tmp.p, tb, keep.p, pos.p, (int)(E + 1), s);
     g_launches++;
     tc::k_orient_off<<<num_sms() * 4, 256, 0, s>>>(g->V, g->off.p, pos.p, p->ooff.p);
     g_launches++;
     int32_t eplus = 0;
-    if ((st = copy_out(&eplus, p->ooff.p + g->V, sizeof(int32_t), s))) return fail(st);
-    if ((st = p->oadj.alloc(eplus))) return fail(st);
+    SP_TRY(copy_out(&eplus, p->ooff.p + g->V, sizeof(int32_t), s));
+    SP_TRY(p->oadj.alloc(eplus));
     if (E > 0) {
       tc::k_orient_scatter<<<num_sms() * 8, 256, 0, s>>>(E, g->adj.p, pos.p, p->oadj.p);
       g_launches++;
     }
     if (cudaStreamSynchronize(s) != cudaSuccess) {
       set_error("tc orientation: %s", cudaGetErrorString(cudaGetLastError()));
-      return fail(SP_ERR_CUDA);
+      return SP_ERR_CUDA;
     }
     p->oriented = true;
   }
@@ -761,19 +763,21 @@ static int build_tc_plan(sp_graph* g) {
     L.adj = p->oriented ? p->oadj.p : g->adj.p;
     L.n = g->V;
     dbuf<int32_t> key, id, skey;
-    if ((st = key.alloc(g->V)) || (st = id.alloc(g->V)) || (st = skey.alloc(g->V)) || (st = p->order.alloc(g->V)))
-      return fail(st);
+    SP_TRY(key.alloc(g->V));
+    SP_TRY(id.alloc(g->V));
+    SP_TRY(skey.alloc(g->V));
+    SP_TRY(p->order.alloc(g->V));
     tc::k_tc_work<<<num_sms() * 8, 256, 0, s>>>(L, key.p, id.p);
     g_launches++;
     size_t tb = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, skey.p, id.p, p->order.p, g->V, 0, 32, s);
     dbuf<unsigned char> tmp;
-    if ((st = tmp.alloc(tb))) return fail(st);
+    SP_TRY(tmp.alloc(tb));
     cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, skey.p, id.p, p->order.p, g->V, 0, 32, s);
     g_launches++;
     if (cudaStreamSynchronize(s) != cudaSuccess) {
       set_error("tc anchor order: %s", cudaGetErrorString(cudaGetLastError()));
-      return fail(SP_ERR_CUDA);
+      return SP_ERR_CUDA;
     }
   }
   p->built = true;
