@@ -1286,7 +1286,9 @@ static int bc_grid(sp_graph* g, const int32_t* d_srcs, int nsrc, int batch_hint,
                    double* sig_out = nullptr, bool push = false) {
   if (bc_direction(g) == 0 && !push) {
     const int batch = std::max(1, std::min(std::min(batch_hint, 64), nsrc));
-    return bc_gather(g, d_srcs, nsrc, batch, batch, 1 << 14, lvl_out, sig_out);
+    const int st = bc_gather(g, d_srcs, nsrc, batch, batch, 1 << 14, lvl_out, sig_out);
+    if (st != SP_ERR_OOM) return st;
+    g->bc->release_state();  // without the memory for in-edges or pieces: push, which needs neither
   }
   BcPlan* p = g->bc;
   cudaStream_t s = g->stream;

@@ -398,7 +398,11 @@ int ensure_reverse(sp_graph* g) {
   T.want(src, E);
   T.want(src_alt, E);
   T.want(temp, t_sort);
-  SP_TRY(T.commit());
+  if (const int st = T.commit()) {
+    g->roff.release();
+    g->radj.release();
+    return st;
+  }
   if (E > 0) {
     SP_CHECK_CUDA(cudaMemcpyAsync(keys.p, g->adj.p, 4 * (size_t)E, cudaMemcpyDeviceToDevice, s));
     k_row_of<<<num_sms() * 8, 256, 0, s>>>(V, E, g->off.p, src.p);

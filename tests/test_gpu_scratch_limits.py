@@ -80,3 +80,34 @@ def test_triangles_when_the_rank_plan_does_not_fit():
             with _only(550 * MB):
                 assert np.array_equal(getattr(dg, call)(), ref), call
             assert np.array_equal(getattr(dg, call)(), ref), call
+
+
+@pytest.mark.parametrize("in_edges", [False, True])
+def test_bc_when_in_edges_or_pieces_do_not_fit(in_edges):
+    # 20 M directed edges on 50,000 vertices: in-edges take 0.4 GB to make and the gather form's
+    # pieces 0.16 GB, where the push form takes 0.1 GB in all
+    import torch
+
+    V = 50000
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    key = torch.unique(torch.randint(V * V, (20_200_000,), generator=gen, device="cuda"))
+    key = key[key // V != key % V]
+    off = torch.searchsorted(key, torch.arange(V + 1, device="cuda") * V).to(torch.int32)
+    adj = (key % V).to(torch.int32)
+    back = torch.sort(key % V * V + key // V).values
+    roff = torch.searchsorted(back, torch.arange(V + 1, device="cuda") * V).to(torch.int32)
+    rev = (roff, (back % V).to(torch.int32)) if in_edges else (None, None)
+    del key, back
+    srcs = np.arange(0, V, 800, dtype=np.int32)
+    with DeviceGraph(off, adj, None, *rev) as dg:
+        ref = dg.bc(srcs).astype(np.float64)
+        lv, sg = dg.bfs_sigma(srcs[:20])
+    with DeviceGraph(off, adj, None, *rev) as dg:
+        with _only((150 if in_edges else 250) * MB):
+            out = dg.bc(srcs).astype(np.float64)
+        assert np.all(np.abs(out - ref) <= 1e-5 * np.abs(ref) + 1e-6)
+        with _only((150 if in_edges else 250) * MB):
+            lv2, sg2 = dg.bfs_sigma(srcs[:20])
+        assert np.array_equal(lv, lv2) and np.array_equal(sg, sg2)
+        again = dg.bc(srcs).astype(np.float64)  # with the memory back
+    assert np.all(np.abs(again - ref) <= 1e-6 * np.abs(ref) + 1e-9)
