@@ -143,9 +143,9 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "sssp.repair"  sp_sssp_dynamic: 1 = a batch with deletions repairs through parents
  *             (weights >= 1), 0 = it solves again from the source, -1 (default) = repair
  *             when the graph's last solve from a source took at least 32 rounds. The
- *             repair pays on high-diameter graphs (grid 1024^2, 100 deletions: 3.7 ms
- *             against 5.3 ms for update + solve) and loses where a solve takes a dozen
- *             rounds (R-MAT 20: 7.9 against 3.9 ms). "sssp.last_marked" (read only):
+ *             repair pays on high-diameter graphs (grid 1024^2, 64 to 100 deletions: 1.5 to
+ *             2.2 ms against 3.8 ms for update + solve) and loses where a solve takes a dozen
+ *             rounds (R-MAT 20: 5.3 against 1.3 ms). "sssp.last_marked" (read only):
  *             vertices the last repair reset (-1: no repair ran).
  *   "sssp.filter"  SSSP: 1 = load dist[u] and send the atomicMin only when the candidate
  *             is lower; 0 = send every atomicMin at once (one L2 round trip less per
@@ -433,7 +433,8 @@ int sp_bc_level_trace(sp_graph_h g, float* records, unsigned long long* times, i
  * bc.hub_deg / bc.hub_chunk, lv.cta_slots), else those knobs and the defaults; -2 the
  * knobs and defaults even with a model; k >= 0 candidate k (to time the table).
  * "<a>.last_variant" (read only): the candidate the last call ran (Louvain: its last
- * level), -1 for knobs and defaults. Counts, distances, levels and path counts are the
+ * level), -1 for knobs and defaults. TC's candidates are the bitmap and hash kernels; the count
+ * in rank order is the default without one of them. Counts, distances, levels and path counts are the
  * same under every candidate; floating-point sums may change grouping. */
 #define SP_VARIANT_PAGERANK 0
 #define SP_VARIANT_TC 1

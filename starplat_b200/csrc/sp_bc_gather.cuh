@@ -27,9 +27,12 @@
 // above hub_deg edges are listed as hub_chunk-edge pieces when their level is formed (the
 // list is kept for the backward sweep), and their partial sums meet in an FP64 scratch.
 //
-// Before and now: R-MAT 20, 256 sources 74.1 -> 23.3 ms; 1000 ER graphs, 16 sources each
-// 81.2 -> 34.7 ms (as one graph instead of a CTA per graph: with a CTA per graph this form
-// took 67 ms); 20 ER graphs of up to 50 thousand vertices, 40 sources each 57 -> 1.9 ms.
+// Push form and this: R-MAT 20, 256 sources 71.2 -> 23.5 ms; 1000 ER graphs, 16 sources each
+// 81.7 -> 33.3 ms (as one graph instead of a CTA per graph: with a CTA per graph this form
+// took 67 ms); 20 ER graphs of up to 50 thousand vertices, 40 sources each 57 -> 1.9 ms; a
+// 300 x 300 grid, one source 9.4 -> 6.3 ms. Slower than the push form: strips of many narrow
+// levels, a team each (20 of 300 x 5 vertices 2.0 -> 2.7 ms, two of 1500 x 4 6.5 -> 12.3), as a
+// level's walk is a longer chain here.
 // What bounds it is the latency of masks and rows (issue 35 % active, L2 75 % hits, 9 GB of
 // DRAM traffic a batch on R-MAT 20, far from its rate).
 #pragma once

@@ -68,8 +68,9 @@ constexpr int SU = 4;                 // 32-edge windows whose loads and atomics
 // 11.5 / 7.9 with 16 (each needs nine V-sized buffers).
 constexpr int BATCH = 8;
 // sp_sssp_dynamic repairs a batch with deletions by default when the graph's last solve
-// took at least this many rounds (100 deletions, the update included: grid 1024^2 repairs in
-// 3.7 ms against 5.3 for a new solve; R-MAT 20, a dozen rounds, 7.9 against 3.9).
+// took at least this many rounds (64 and 100 deletions, weights 1 to 100, the update included:
+// grid 1024^2 repairs in 2.2 and 1.5 ms against 3.8 for a new solve; R-MAT 20, a dozen rounds, 5.3
+// against 1.3).
 constexpr int REPAIR_MIN_ROUNDS = 32;
 constexpr unsigned FULL = 0xffffffffu;
 
@@ -588,8 +589,8 @@ __device__ int epoch_choice(const Args& a, float fn, float rounds_prev, float re
 // every step's marks, counters and far pushes waited for in the step, and rows loaded when
 // popped, a cascade step took 5,500 cycles for 25 to 35 edges on the grid, and an R-MAT
 // step issued one counter atomic and mostly idle passes per 128 edges. Now (rings, bit
-// windows, rows beside the atomicMins, four lanes to a row): grid 4096^2 28.9 -> 16.8 ms,
-// R-MAT 23 6.98 -> 3.58 ms (13 rounds, 330 M edges relaxed), ER 2^20 2.2 -> 1.1 ms, grid
+// windows, rows beside the atomicMins, four lanes to a row): grid 4096^2 31.3 -> 18.0 ms,
+// R-MAT 23 6.9 -> 3.3 ms (13 rounds, 330 M edges relaxed), ER 2^20 2.2 -> 1.1 ms, grid
 // 300^2 1.44 -> 0.93 ms.
 __device__ __forceinline__ void delta_run(const Args& a, const int blk, const int nblk, RingMem* ring) {
   Ctl* c = a.ctl;
@@ -1421,7 +1422,7 @@ static int sssp_schedule(sp_graph* g, int64_t& delta, int& ctas, int& local) {
     // learned schedule: score every candidate, run the best (fixed heuristic if no
     // model). The cascade budget is a candidate too unless the sssp.local knob is set.
     static const double mults[] = {1, 2, 4, 8, 16, 32, 64};
-    static const int cts[] = {1, 2, 4};
+    static const int cts[] = {1, 2, 4};  // 4: as many as are resident (ss::CTAS); the model knows it as 4
     // cascade budgets: off, the default, and a long one (grid 4096^2: 30.8 ms at 64,
     // 28.8 at 256 with the same width and CTAs)
     const int locs[3] = {0, ss::LOCAL_STEPS, 4 * ss::LOCAL_STEPS};

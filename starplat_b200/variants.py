@@ -4,7 +4,8 @@ Each of these algorithms has a small table of kernel variants in the library
 (sp_variant_count): PageRank chooses which of the most-gathered sources allocate their
 contrib gathers in L1, the srcList cache policy and the load width; TC chooses the
 shared-bitmap kernel's CTA width (up to 65536 vertices) or the hash kernel's probe-list
-elements per lane (above); BC chooses the degree above which a level-list entry is cut
+elements per lane (above; without a model larger symmetric graphs are counted in rank order,
+which is no candidate); BC chooses the degree above which a level-list entry is cut
 into pieces shared by all warps, and the piece size; Louvain chooses, at every level,
 the shared-memory table size of its CTA degree bin. Variants change only how work is
 split or cached: counts, levels and path counts are the same under every one of them.
