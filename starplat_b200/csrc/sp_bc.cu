@@ -1652,8 +1652,8 @@ namespace sp {
 // takes about 14 us in the union and 8 in a team, an entry (a source's visit to a vertex)
 // 0.6 ns and 90, and a grid has about 2 sqrt(V) levels (a strip more, which favours teams
 // further: hence the quarter in their favour). As one graph / as teams, ms: 20 strips of
-// 300 x 5, 4 sources 6.0 / 2.9; 2 of 1500 x 4 19.5 / 13.1; 200 grids of 60 x 60, 4 sources 3.6 / 2.6;
-// 50 of 100 x 100 4.9 / 5.0; 10 of 200 x 200, 16 sources 10 / 57.
+// 300 x 5, 4 sources 6.0 / 2.5; 2 of 1500 x 4 19.5 / 11.4; 200 grids of 60 x 60, 4 sources 3.6 / 2.4;
+// 50 of 100 x 100 4.8 / 4.9; 10 of 200 x 200, 16 sources 10 / 54.
 static bool bc_teams_faster(sp_graph* g, int ngraphs, const std::vector<int32_t>& voff,
                             const std::vector<int32_t>& soff) {
   if (g->symmetric != 1 || g->max_out_deg < 0 || g->max_out_deg > bc::NARROW_DEG) return false;

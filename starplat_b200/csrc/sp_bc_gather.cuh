@@ -31,7 +31,7 @@
 // 81.7 -> 33.3 ms (as one graph instead of a CTA per graph: with a CTA per graph this form
 // took 67 ms); 20 ER graphs of up to 50 thousand vertices, 40 sources each 57 -> 1.9 ms; a
 // 300 x 300 grid, one source 9.4 -> 6.3 ms. Slower than the push form: strips of many narrow
-// levels, a team each (20 of 300 x 5 vertices 2.0 -> 2.7 ms, two of 1500 x 4 6.5 -> 12.3), as a
+// levels, a team each (20 of 300 x 5 vertices 2.0 -> 2.5 ms, two of 1500 x 4 6.5 -> 11.4), as a
 // level's walk is a longer chain here.
 // What bounds it is the latency of masks and rows (issue 35 % active, L2 75 % hits, 9 GB of
 // DRAM traffic a batch on R-MAT 20, far from its rate).
@@ -198,16 +198,21 @@ __device__ __forceinline__ void put_delta(const Gather& G, int v, unsigned long 
   double sum = 0.0;
   const unsigned nib = own_bits<SW>(m, sl);
   double* r = G.row + (size_t)v * SW;
+  // every load before the first store, which the compiler could not move them across
+  double s[4], before = 0.0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s[j] = (nib >> j) & 1u ? r[own_at<SW>(sl, j)] : 1.0;
+  if (sl == 0 && m) before = G.bc[v];
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     if ((nib >> j) & 1u) {
-      const double s = r[own_at<SW>(sl, j)], d = s * acc[j];
-      r[own_at<SW>(sl, j)] = (1.0 + d) / s;
+      const double d = s[j] * acc[j];
+      r[own_at<SW>(sl, j)] = (1.0 + d) / s[j];
       sum += d;
     }
 #pragma unroll
   for (int o = SW / 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if (sl == 0 && sum != 0.0) G.bc[v] += sum;
+  if (sl == 0 && sum != 0.0) G.bc[v] = before + sum;
 }
 
 template <int SW>
