@@ -58,12 +58,15 @@ constexpr int HUB_CHUNK = 64;
 constexpr int WIDE_HUB_DEG = 256, WIDE_HUB_CHUNK = 128;
 constexpr double WIDE_E = 12e6;
 constexpr int NARROW_DEG = 8;
-// Levels and path counts on a graph without in-edges: a first call of up to this many entries
-// times sources pushes, as the in-edges that the gather form needs cost more than it gains.
-// One source, first call pushing / gathering: directed R-MAT 14 (175 thousand entries) 0.27 / 0.41
-// ms, 17 (1.9 M) 0.45 / 0.58, R-MAT 17 (3.6 M) 0.46 / 0.50; 16 sources, directed 14 0.44 / 0.51,
-// 17 0.95 / 0.92, R-MAT 17 1.16 / 0.90.
+// Levels and path counts of up to 16 sources on a graph without in-edges: a first call of up to
+// this many entries times sources pushes, as the in-edges that the gather form needs cost more
+// than it gains.
+// One source, first call pushing / gathering: directed R-MAT 14 (175 thousand entries) 0.23 / 0.41
+// ms, 17 (1.9 M) 0.34 / 0.58, R-MAT 17 (3.6 M) 0.36 / 0.50; 16 sources, directed 14 0.34 / 0.51,
+// 17 0.93 / 0.92, R-MAT 17 1.16 / 0.90. On a directed graph, whose gather walks two rows an entry,
+// such calls push every time: 16 sources on R-MAT 14 0.32 / 0.40, one on ER 30,000 of degree 4 0.29 / 0.38.
 constexpr int64_t PUSH_MAX_E = 8000000;
+constexpr int32_t PUSH_MAX_V = 1 << 18;  // its rows take 900 bytes a vertex
 constexpr int CLUSTER_DEFAULT = 1;  // CTAs per graph in the many-graphs form (bc.cluster)
 // Successors whose loads are in flight together in the backward sweep (measured when
 // each successor cost a sigma and a delta load),
@@ -1024,9 +1027,11 @@ struct BcPlan {
   int64_t vmax = 0, vsq = 0, vrows[4] = {}, vedges[4] = {};
   int var_choice = -1, var_nsrc = 0;
   unsigned var_gen = 0;
-  // Gives back the gather form's rows, masks and lists.
+  // Gives back the rows, masks and lists of a form that did not fit.
   void release_state() {
     sigma.release();
+    delta.release();
+    q.release();
     dacc.release();
     masks.release();
     flv.release();
@@ -1769,9 +1774,15 @@ int bc_levels(sp_graph* g, const int32_t* d_srcs, int nsrc, int32_t* lvl_out, do
     return SP_OK;
   };
   SP_TRY(clear());
-  const bool push = !g->bc->levels_ran && !g->has_rev && g->symmetric < 0 && g->E * nsrc <= bc::PUSH_MAX_E;
+  const int64_t size = g->E * nsrc;
+  const bool push = nsrc <= 16 && g->V <= bc::PUSH_MAX_V && size <= bc::PUSH_MAX_E &&
+                    (g->symmetric == 0 || (g->symmetric < 0 && !g->has_rev && !g->bc->levels_ran));
   g->bc->levels_ran = true;
-  int st = bc_grid(g, d_srcs, nsrc, 64, lvl_out, sig_out, push);
+  int st = push ? bc_grid(g, d_srcs, nsrc, nsrc, lvl_out, sig_out, true) : SP_ERR_OOM;
+  if (st == SP_ERR_OOM) {
+    if (push) g->bc->release_state();  // the gather form's rows are smaller
+    st = bc_grid(g, d_srcs, nsrc, 64, lvl_out, sig_out);
+  }
   if (st != SP_ERR_UNSUPPORTED || nsrc <= 16) return st;
   SP_TRY(clear());
   for (int k = 0; k < nsrc; k += 16)

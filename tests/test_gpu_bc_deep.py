@@ -73,8 +73,9 @@ def test_many_deep_graphs(shape, counts):
 @pytest.mark.parametrize("directed", [False, True])
 @pytest.mark.parametrize("nsrc", [1, 16, 64])
 def test_levels_without_in_edges(directed, nsrc):
-    # a first call of few sources needs no in-edges, later ones and larger calls (8 M entries
-    # times sources) make them: the same levels and path counts
+    # a call of few sources on a directed graph, and a first one on any graph without in-edges,
+    # pushes; other calls (from 17 sources or 8 M entries times sources) gather: the same levels
+    # and path counts
     g = G.rmat(15, 8, seed=5, directed=directed)
     assert (g.E * nsrc > 8_000_000) == (nsrc == 64)
     srcs = G.pick_sources(g, nsrc, seed=2, min_out_degree=0)

@@ -111,3 +111,14 @@ def test_bc_when_in_edges_or_pieces_do_not_fit(in_edges):
         assert np.array_equal(lv, lv2) and np.array_equal(sg, sg2)
         again = dg.bc(srcs).astype(np.float64)  # with the memory back
     assert np.all(np.abs(again - ref) <= 1e-6 * np.abs(ref) + 1e-9)
+
+
+def test_first_levels_when_the_push_form_does_not_fit():
+    # without in-edges a first call pushes, in rows of 235 MB here; the gather form takes 60
+    g = G.grid(512, 512)
+    with DeviceGraph(g.indexofNodes, g.edgeList, None, None, None) as dg:
+        ref = dg.bfs_sigma(np.array([70000], np.int32))
+    with DeviceGraph(g.indexofNodes, g.edgeList, None, None, None) as dg:
+        with _only(150 * MB):
+            out = dg.bfs_sigma(np.array([70000], np.int32))
+    assert np.array_equal(out[0], ref[0]) and np.all(np.abs(out[1] - ref[1]) <= 1e-12 * ref[1])
