@@ -143,9 +143,9 @@ int sp_graph_info(sp_graph_h g, int32_t* V, int64_t* E, int32_t* symmetric);
  *   "sssp.repair"  sp_sssp_dynamic: 1 = a batch with deletions repairs through parents
  *             (weights >= 1), 0 = it solves again from the source, -1 (default) = repair
  *             when the graph's last solve from a source took at least 32 rounds. The
- *             repair pays on high-diameter graphs (grid 1024^2, 64 to 100 deletions: 1.5 to
- *             2.2 ms against 3.8 ms for update + solve) and loses where a solve takes a dozen
- *             rounds (R-MAT 20: 5.3 against 1.3 ms). "sssp.last_marked" (read only):
+ *             repair pays on high-diameter graphs (grid 1024^2, 64 deletions: 1.0 to 1.3 ms
+ *             against 5.2 ms for update + solve) and loses where a solve takes a dozen
+ *             rounds (R-MAT 20: 3.3 against 1.7 ms). "sssp.last_marked" (read only):
  *             vertices the last repair reset (-1: no repair ran).
  *   "sssp.filter"  SSSP: 1 = load dist[u] and send the atomicMin only when the candidate
  *             is lower; 0 = send every atomicMin at once (one L2 round trip less per

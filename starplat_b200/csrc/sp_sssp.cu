@@ -68,9 +68,9 @@ constexpr int SU = 4;                 // 32-edge windows whose loads and atomics
 // 11.5 / 7.9 with 16 (each needs nine V-sized buffers).
 constexpr int BATCH = 8;
 // sp_sssp_dynamic repairs a batch with deletions by default when the graph's last solve
-// took at least this many rounds (64 and 100 deletions, weights 1 to 100, the update included:
-// grid 1024^2 repairs in 2.2 and 1.5 ms against 3.8 for a new solve; R-MAT 20, a dozen rounds, 5.3
-// against 1.3).
+// took at least this many rounds (64 deletions, the update included, as the benchmark times
+// them: grid 1024^2, weights to 1000, repairs in 1.0 to 1.3 ms against 5.2 for a new solve;
+// directed R-MAT 20, a dozen rounds, 3.3 against 1.7).
 constexpr int REPAIR_MIN_ROUNDS = 32;
 constexpr unsigned FULL = 0xffffffffu;
 
